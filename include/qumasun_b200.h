@@ -157,14 +157,14 @@ int qg_hamiltonian_apply_z(qg_hamiltonian ham, int ns, const double* X, long lon
  * 3 doubles each, bohr^-1), nsk states per k-point, state s of k-point k at
  * X + k*ldk + s*ldx (HX + k*ldkh + s*ldhx), DEVICE FP64, ldx/ldhx >= 2N,
  * ldk >= nsk*ldx. Each stencil work item and projector block carries its k-point's
- * coefficients and Bloch tables, so all k-points share one launch per phase. The
+ * coefficients and phases, so all k-points share one launch per phase. The
  * operator's own k-vector (qg_hamiltonian_set_kvector) is not used. No counterpart in
  * the reference, which loops over k (qumasun_kpoint.lobpcg.h:25-41). */
 int qg_hamiltonian_apply_zk(qg_hamiltonian ham, int nk, const double* kvecs, int nsk, const double* X,
                             long long ldx, long long ldk, double* HX, long long ldhx, long long ldkh);
 /* Complex64 states (FP32 {re[N], im[N]} per state): the same operator with FP32
- * stencil, potential, Bloch tables and projector sums (the FP32 counterpart of
- * qg_hamiltonian_apply_f for k-points); single k-vector / several k-points. */
+ * stencil and potential; the projector sums are FP64 (single k-vector / several
+ * k-points). */
 int qg_hamiltonian_apply_zf(qg_hamiltonian ham, int ns, const float* X, long long ldx, float* HX, long long ldhx);
 int qg_hamiltonian_apply_zkf(qg_hamiltonian ham, int nk, const double* kvecs, int nsk, const float* X,
                              long long ldx, long long ldk, float* HX, long long ldhx, long long ldkh);
@@ -391,14 +391,16 @@ int qg_hegv_small_batched_z(qg_context ctx, int batch, int k, const double* A, c
  * global memory (2-5 fall back as 0 does where the shape does not fit). All give the same bits. Complex states use the one-plane ring kernel
  * unless 1 is set. */
 int qg_hamiltonian_set_stencil_kernel(qg_hamiltonian ham, int variant);
-/* Tuning of the nonlocal passes: states per projection block (1, 2, 4, 8 or 16;
- * complex states use at most 4), states per scatter group of the real apply (4 or
- * 8), and blocks per atom in the projection (1-8, one thread-block cluster; the
- * engine's choice follows the cell alone: 1 for cells of more than 16 atoms, else
- * one per 4096 sphere points of the largest atom); 0 = the
- * engine's choice. The block sizes do not change the result (same sums in the same
- * order); the parts per atom change the summation order of the projections (last
- * bits only), and the engine's choice never depends on the number of states. */
+/* Tuning of the nonlocal passes of real states: states per block of the atom-by-atom
+ * projection (1, 2, 4, 8 or 16), states per scatter group (4 or 8), and blocks per atom
+ * in the projection (1-8, one thread-block cluster); 0 = the engine's choice, which
+ * follows the cell and the type alone: atom by atom with one block per 4096 sphere points of
+ * the largest atom for cells of at most 16 atoms and for FP32 states (1 block above 16
+ * atoms), brick by brick on the FP64 tensor cores for FP64 states of larger cells.
+ * The block sizes do not change the result (same sums in the same order); the parts per
+ * atom change the summation order of the projections (last bits only), and the engine's
+ * choice never depends on the number of states. Complex states always go brick by
+ * brick and ignore the three values. */
 int qg_hamiltonian_set_nonlocal_blocking(qg_hamiltonian ham, int project_states, int scatter_states,
                                          int project_parts);
 /* Real-state LOBPCG (qg_lobpcg_d, _device, cells) with more than 128 Gram columns: 1

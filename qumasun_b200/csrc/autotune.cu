@@ -15,6 +15,7 @@
 #include <cfloat>
 #include <vector>
 
+#include "nonlocal.h"
 #include "qg_internal.h"
 #include "stencil_common.cuh"
 
@@ -24,11 +25,8 @@ template <typename T>
 int timed_phases(qg_hamiltonian h, int ns, const T* X, long long ldx, T* HX, long long ldhx, int reps,
                  float best[3]) {
     best[0] = best[1] = best[2] = FLT_MAX;
-    T* coef = nullptr;
-    if (h->pj.na > 0) {
-        QG_TRY(h->coef.reserve(qg::coef_scratch_elems(h, ns) * sizeof(T)));
-        coef = h->coef.as<T>();
-    }
+    QG_TRY(h->coef.reserve(qg::nonlocal_scratch(h, 1, ns, false) * sizeof(double)));
+    void* coef = h->coef.ptr;
     for (int r = 0; r < reps + 1; ++r) {  // the first apply warms caches and the instruction path
         qg::PhaseTimer pt;
         QG_TRY(qg::apply_hamiltonian<T>(h, ns, X, ldx, HX, ldhx, coef, h->ctx->stream, &pt));

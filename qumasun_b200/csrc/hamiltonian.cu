@@ -1,15 +1,15 @@
 // Kohn-Sham H|psi> on the device (mHamiltonianMatrix_ddm, qumasun_mpi.matrix.h:20-43):
 //   H psi = V psi + sum_atoms sum_k E_k sum_m |p_km> dV <p_km|psi> - 1/2 Lap psi.
 //
-// Main path (shapes the TMA kernel accepts), three launches for a block of states:
-//   k_project     c[a,ch][s] = E_ch dV sum_{p in sphere(a)} tab[ch][p] psi_s[g(p)]
+// Three steps for a block of states:
+//   projection    c[a,ch][s] = E_ch dV sum_{p in sphere(a)} tab[ch][p] psi_s[g(p)]
 //                 (InnerProd_1S_1R / InnerProd_2S_1R of ProjectionPP, PseudoPotOperator.h:740-772,
-//                 all atoms, channels and states at once);
-//   k_stencil_tma H psi = V psi - 1/2 Lap psi (stencil_tma.cu: persistent, TMA-staged);
+//                 all atoms, channels and states at once): k_project, atom by atom, or the bricks of
+//                 nonlocal.cu;
+//   stencil       H psi = V psi - 1/2 Lap psi: the ring kernels (stencil_*.cu), or k_hamiltonian, a
+//                 register-window kernel for any shape;
 //   k_scatter_all H psi[s][g] += sum_{entries e of g} sum_ch val[e][ch] c[a_e,ch][s]
 //                 (Add_1S / Add_2S of ProjectionPP turned into a per-point gather, no atomics).
-// Fallback path (any shape): k_project, then k_hamiltonian, a register-window
-// stencil kernel with the per-point scatter fused in.
 //
 // k_hamiltonian data flow (per thread block: SPB states, ty full x-rows, a slab of z):
 // the block marches up z; each thread keeps its own column's 2R+1 z-values in
@@ -24,6 +24,7 @@
 
 #include <cooperative_groups.h>
 
+#include "nonlocal.h"
 #include "qg_internal.h"
 #include "stencil_common.cuh"
 #include "precond.h"
@@ -160,27 +161,11 @@ __global__ void __launch_bounds__(1024) k_hamiltonian(const HamArgs<T> a) {
 
         const long long gi = zoff + col;
         const T vloc = a.V[gi];
-        T nl[SPB];
-#pragma unroll
-        for (int s = 0; s < SPB; ++s) nl[s] = T(0);
-        if (a.row) {
-            const int e0 = a.row[gi], e1 = a.row[gi + 1];
-            for (int e = e0; e < e1; ++e) {
-                const int at = a.ent_atom[e];
-                const T* ev = a.ent_val + (long long)e * a.nch;
-                for (int ch = 0; ch < a.nch; ++ch) {
-                    const T tv = ev[ch];
-#pragma unroll
-                    for (int s = 0; s < SPB; ++s)
-                        nl[s] += tv * a.coef[(long long)(at * a.nch + ch) * a.ldc + (valid[s] ? s0 + s : s0)];
-                }
-            }
-        }
 #pragma unroll
         for (int s = 0; s < SPB; ++s) {
             const T* pc = sm + s * rows * W + (R + ly) * W + R + ix;
             const T lap = stencil_point<T, ORDER, R>(pc, W, q[s], a);
-            const T out = (vloc * q[s][R] + nl[s]) + lap;
+            const T out = vloc * q[s][R] + lap;
             if (valid[s]) a.HX[(long long)(s0 + s) * a.ldhx + gi] = out;
         }
         __syncthreads();
@@ -596,12 +581,6 @@ size_t coef_scratch_elems(qg_hamiltonian h, int ns) {
     return (size_t)coef_ld(ns) * pj.na * pj.nch;
 }
 
-size_t coef_scratch_elems_z(qg_hamiltonian h, int nk, int nsk) {
-    const DevProjectors& pj = h->pj;
-    if (pj.na <= 0 || pj.nch <= 0) return 0;
-    return (size_t)2 * nk * coef_ld(nsk) * pj.na * pj.nch;
-}
-
 // Stencil kernel for a real-state apply: the forced variant when it accepts the shape,
 // else the two-row ring kernel -- FP64 with V in the ring (4), FP32 with V from global
 // memory (5) -- measured on the 80^3 cell, 256 states (whole apply, order 2/4/6/8):
@@ -631,7 +610,7 @@ static int ring_stencil_variant(qg_hamiltonian h, const HamArgs<T>& a) {
 
 template <typename T>
 int apply_hamiltonian(qg_hamiltonian h, int ns, const T* X, long long ldx, T* HX, long long ldhx,
-                      T* coef, cudaStream_t st, PhaseTimer* pt) {
+                      void* scratch, cudaStream_t st, PhaseTimer* pt, bool atom_major) {
     const DevProjectors& pj = h->pj;
     HamArgs<T> a{};
     a.X = X; a.ldx = ldx; a.HX = HX; a.ldhx = ldhx; a.ns = ns;
@@ -681,61 +660,44 @@ int apply_hamiltonian(qg_hamiltonian h, int ns, const T* X, long long ldx, T* HX
     const bool nonlocal = pj.na > 0 && pj.nch > 0;
     const long long N = h->N();
     const int variant = ring_stencil_variant<T>(h, a);
-    if (variant != 1) {
-        auto stencil = [&]() {
-            if (variant == 3) return launch_stencil_pair<T>(a, h->order, st);
-            if (variant == 4) return launch_stencil_rows<T>(a, h->order, st, true);
-            if (variant == 5) return launch_stencil_rows<T>(a, h->order, st, false);
-            return launch_stencil_tma<T>(a, h->order, st);
-        };
-        if (!nonlocal) {
-            if (pt) pt->mark(1, st);
-            QG_TRY(stencil());
-            QG_CUDA_TRY(cudaGetLastError());
-            if (pt) pt->mark(-1, st);
-            return QG_OK;
+    T* coef = static_cast<T*>(scratch);
+    if (pt) pt->mark(nonlocal ? 0 : 1, st);
+    if (nonlocal) {
+        // FP32 states, a forced split of the atoms and the no-allocation entry point go atom by atom
+        bool bricks = !atom_major && h->proj_parts == 0 && bricks_for_real(pj);
+        if constexpr (sizeof(T) == 8) {
+            if (bricks)
+                QG_TRY(brick_project<T>(h, 1, ns, false, X, ldx, 0, nullptr, pj.ch_scale, coef,
+                                        coef + coef_elems(h, 1, ns, false), st));
+        } else {
+            bricks = false;
         }
-        // projection of all states, persistent stencil + V, then the nonlocal scatter
-        if (pt) pt->mark(0, st);
-        QG_TRY(launch_project<T>(pj, ns, X, ldx, coef, coef_ld(ns), h->proj_sb, h->proj_parts, st));
+        if (!bricks) QG_TRY(launch_project<T>(pj, ns, X, ldx, coef, coef_ld(ns), h->proj_sb, h->proj_parts, st));
         if (pt) pt->mark(1, st);
-        QG_TRY(stencil());
+    }
+    int rc;
+    if (variant == 3) rc = launch_stencil_pair<T>(a, h->order, st);
+    else if (variant == 4) rc = launch_stencil_rows<T>(a, h->order, st, true);
+    else if (variant == 5) rc = launch_stencil_rows<T>(a, h->order, st, false);
+    else if (variant == 2) rc = launch_stencil_tma<T>(a, h->order, st);
+    else if (h->order == 2) rc = launch_stencil<T, 2>(a, h->nz, st);
+    else if (h->order == 4) rc = launch_stencil<T, 4>(a, h->nz, st);
+    else if (h->order == 6) rc = launch_stencil<T, 6>(a, h->nz, st);
+    else rc = launch_stencil<T, 8>(a, h->nz, st);
+    QG_TRY(rc);
+    if (nonlocal) {
         if (pt) pt->mark(2, st);
         QG_TRY(launch_scatter_all<T>(pj, HX, ldhx, ns, N, coef, coef_ld(ns), h->scatter_sg, st));
-        if (pt) pt->mark(-1, st);
-        QG_CUDA_TRY(cudaGetLastError());
-        return QG_OK;
     }
-    // register-window kernel with the nonlocal scatter fused per point
-    if (pt) pt->mark(0, st);
-    if (nonlocal) {
-        QG_TRY(launch_project<T>(pj, ns, X, ldx, coef, coef_ld(ns), h->proj_sb, h->proj_parts, st));
-        a.row = pj.row;
-        a.ent_atom = pj.ent_atom;
-        if constexpr (sizeof(T) == 8) a.ent_val = reinterpret_cast<const T*>(pj.ent_val_d);
-        else a.ent_val = reinterpret_cast<const T*>(pj.ent_val_f);
-        a.nch = pj.nch;
-        a.ldc = coef_ld(ns);
-        a.coef = coef;
-    }
-    if (pt) pt->mark(1, st);
-    int rc;
-    switch (h->order) {
-        case 2: rc = launch_stencil<T, 2>(a, h->nz, st); break;
-        case 4: rc = launch_stencil<T, 4>(a, h->nz, st); break;
-        case 6: rc = launch_stencil<T, 6>(a, h->nz, st); break;
-        default: rc = launch_stencil<T, 8>(a, h->nz, st); break;
-    }
-    if (rc != QG_OK) return rc;
     if (pt) pt->mark(-1, st);
     QG_CUDA_TRY(cudaGetLastError());
     return QG_OK;
 }
 
 template int apply_hamiltonian<double>(qg_hamiltonian, int, const double*, long long, double*,
-                                       long long, double*, cudaStream_t, PhaseTimer*);
+                                       long long, void*, cudaStream_t, PhaseTimer*, bool);
 template int apply_hamiltonian<float>(qg_hamiltonian, int, const float*, long long, float*,
-                                      long long, float*, cudaStream_t, PhaseTimer*);
+                                      long long, void*, cudaStream_t, PhaseTimer*, bool);
 
 }  // namespace qg
 
@@ -761,8 +723,8 @@ int upload(T** dst, const std::vector<T>& src) {
 void free_projectors(DevProjectors& pj) {
     cudaFree(pj.atom_off); cudaFree(pj.pt_g); cudaFree(pj.tab_d); cudaFree(pj.tab_f);
     cudaFree(pj.ch_scale); cudaFree(pj.ch_dv); cudaFree(pj.ch_E); cudaFree(pj.row); cudaFree(pj.ent_atom); cudaFree(pj.ent_val_d);
-    cudaFree(pj.ent_val_f); cudaFree(pj.pt_u); cudaFree(pj.ent_pt); cudaFree(pj.ztab); cudaFree(pj.zent);
-    cudaFree(pj.ztab_f); cudaFree(pj.zent_f);
+    cudaFree(pj.ent_val_f);
+    qg::free_bricks(pj.bricks);
     pj = DevProjectors();
 }
 
@@ -852,13 +814,12 @@ int build_projectors(qg_hamiltonian h, const qg_hamiltonian_desc* d) {
     for (long long p = 0; p < npts; ++p) row[pt_g[p] + 1]++;
     for (long long g = 0; g < N; ++g) row[g + 1] += row[g];
     std::vector<int> fill(row.begin(), row.end() - 1);
-    std::vector<int> ent_atom(npts), ent_pt(npts);
+    std::vector<int> ent_atom(npts);
     std::vector<double> ent_val((size_t)npts * nch);
     for (int a = 0; a < na; ++a)
         for (int p = atom_off[a]; p < atom_off[a + 1]; ++p) {
             const int e = fill[pt_g[p]]++;
             ent_atom[e] = a;
-            ent_pt[e] = p;
             for (int ch = 0; ch < nch; ++ch) ent_val[(size_t)e * nch + ch] = tab_d[(size_t)ch * npts + p];
         }
     std::vector<float> ent_val_f(ent_val.begin(), ent_val.end());
@@ -878,9 +839,7 @@ int build_projectors(qg_hamiltonian h, const qg_hamiltonian_desc* d) {
     QG_TRY(upload(&pj.ent_atom, ent_atom));
     QG_TRY(upload(&pj.ent_val_d, ent_val));
     QG_TRY(upload(&pj.ent_val_f, ent_val_f));
-    QG_TRY(upload(&pj.pt_u, pt_u));
-    QG_TRY(upload(&pj.ent_pt, ent_pt));
-    return QG_OK;
+    return qg::build_bricks(h, atom_off, pt_u, tabs);
 }
 
 void destroy_ham(qg_hamiltonian h) {
@@ -965,12 +924,8 @@ static int apply_device(qg_hamiltonian h, int ns, const T* X, long long ldx, T* 
     if (ldx < N || ldhx < N) return QG_ERR_INVALID;
     if (h->gx != 0.0 || h->gy != 0.0 || h->gz != 0.0) return QG_ERR_INVALID;
     QG_CUDA_TRY(cudaSetDevice(h->ctx->device));
-    T* coef = nullptr;
-    if (h->pj.na > 0) {
-        QG_TRY(h->coef.reserve(qg::coef_scratch_elems(h, ns) * sizeof(T)));
-        coef = h->coef.as<T>();
-    }
-    return qg::apply_hamiltonian<T>(h, ns, X, ldx, HX, ldhx, coef, h->ctx->stream);
+    QG_TRY(h->coef.reserve(qg::nonlocal_scratch(h, 1, ns, false) * sizeof(double)));
+    return qg::apply_hamiltonian<T>(h, ns, X, ldx, HX, ldhx, h->coef.ptr, h->ctx->stream);
 }
 
 namespace qg {
@@ -1054,13 +1009,9 @@ int qg_hamiltonian_apply_timed_d(qg_hamiltonian h, int ns, const double* X, long
     const long long N = h->N();
     if (ldx < N || ldhx < N) return QG_ERR_INVALID;
     QG_CUDA_TRY(cudaSetDevice(h->ctx->device));
-    double* coef = nullptr;
-    if (h->pj.na > 0) {
-        QG_TRY(h->coef.reserve(qg::coef_scratch_elems(h, ns) * sizeof(double)));
-        coef = h->coef.as<double>();
-    }
+    QG_TRY(h->coef.reserve(qg::nonlocal_scratch(h, 1, ns, false) * sizeof(double)));
     qg::PhaseTimer pt;
-    const int rc = qg::apply_hamiltonian<double>(h, ns, X, ldx, HX, ldhx, coef, h->ctx->stream, &pt);
+    const int rc = qg::apply_hamiltonian<double>(h, ns, X, ldx, HX, ldhx, h->coef.ptr, h->ctx->stream, &pt);
     if (rc != QG_OK) return rc;
     pt.totals(ms_phases);
     QG_CUDA_TRY(cudaGetLastError());
@@ -1097,14 +1048,9 @@ int qg_hamiltonian_launches_per_apply(qg_hamiltonian h, int ns) {
     if (!h || ns < 0) return QG_ERR_INVALID;
     if (ns == 0) return 0;
     const bool nonlocal = h->pj.na > 0 && h->pj.nch > 0;
-    qg::HamArgs<double> a{};
-    a.X = reinterpret_cast<const double*>(16); a.HX = reinterpret_cast<double*>(16); a.V = h->V_d;
-    a.ldx = a.ldhx = h->N(); a.nx = h->nx; a.ny = h->ny; a.nz = h->nz; a.err = h->ctx->dev_status;
-    if (qg::ring_stencil_variant<double>(h, a) != 1) {
-        if (!nonlocal) return 1;
-        return 3;  // projection, stencil + V, nonlocal scatter
-    }
-    return (nonlocal ? 1 : 0) + 1;
+    if (!nonlocal) return 1;
+    // projection, stencil + V, nonlocal scatter
+    return (h->proj_parts == 0 && qg::bricks_for_real(h->pj) ? qg::brick_project_launches(h, ns) : 1) + 2;
 }
 
 int qg_hamiltonian_apply_host_d(qg_hamiltonian h, int ns, const double* X, double* HX) {

@@ -34,6 +34,7 @@
 #include "gram_mixed.h"
 #include "gram_split.h"
 #include "gram_ts.h"
+#include "nonlocal.h"
 #include "precond.h"
 #include "qg_internal.h"
 #include "small_eig.h"
@@ -458,8 +459,7 @@ struct Solver {
             lwork = std::max(lwork, lw2);
             QG_TRY(work.reserve((size_t)std::max(lwork, 1) * sizeof(cuDoubleComplex)));
         }
-        QG_TRY(h->coef.reserve((c == 1 ? qg::coef_scratch_elems(h, n) : qg::coef_scratch_elems_z(h, 1, n)) *
-                               sizeof(double)));
+        QG_TRY(h->coef.reserve(qg::nonlocal_scratch(h, 1, n, c == 2) * sizeof(double)));
         if (mixed) QG_TRY(mg.setup(N, (int)g3, mixed_pieces));
         if (i8 && c == 1) QG_TRY(mg.setup(N, (int)g3, qg::kI8Slices));
         if (c == 1) {
@@ -1149,7 +1149,7 @@ int run_lobpcg_zk(qg_hamiltonian h, const qg_lobpcg_options* opt, int nk, const 
         s.lwork = std::max(lw1, lw2);
         QG_TRY(s.work.reserve((size_t)std::max(s.lwork, 1) * sizeof(cuDoubleComplex)));
     }
-    QG_TRY(h->coef.reserve(qg::coef_scratch_elems_z(h, nk, nb) * sizeof(double)));
+    QG_TRY(h->coef.reserve(qg::nonlocal_scratch(h, nk, nb, true) * sizeof(double)));
     // pencils of up to kSmallHegMax rows: all k-points' Hermitian pencils in one launch
     // of the one-block Jacobi solver (small_eig.cu), cuSOLVER's zhegvd per k-point
     // otherwise and for any pencil the Jacobi solver rejects

@@ -68,7 +68,7 @@ int qg_hamiltonian_apply_noalloc_d(qg_hamiltonian h, int ns, const double* X, lo
     QG_CUDA_TRY(cudaSetDevice(h->ctx->device));
     double* coef = nullptr;
     QG_TRY(coef_address(h->ctx->device, &coef));
-    return qg::apply_hamiltonian<double>(h, ns, X, ldx, HX, ldhx, coef, h->ctx->stream);
+    return qg::apply_hamiltonian<double>(h, ns, X, ldx, HX, ldhx, coef, h->ctx->stream, nullptr, true);
 }
 
 }  // extern "C"

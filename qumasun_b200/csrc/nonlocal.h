@@ -1,0 +1,47 @@
+// Nonlocal projectors as FP64 tensor-core contractions over bricks of the grid (nonlocal.cu).
+#pragma once
+#include <vector>
+
+#include "qg_internal.h"
+
+namespace qg {
+
+// Sphere points of one geometry as the builder takes them: atom a owns the points
+// [atom_off[a], atom_off[a+1]), u = 3 unwrapped grid coordinates per point (rows of
+// consecutive x one after another), tabs[ch][p] the channel values.
+int build_bricks(qg_hamiltonian h, const std::vector<int>& atom_off, const std::vector<int>& u,
+                 const std::vector<std::vector<double>>& tabs);
+void free_bricks(BrickTables& b);
+
+// Rows of projector coefficients per k-point: the state count rounded up to 16 (real), or
+// {re, im} in alternating groups of 8 (complex).
+inline long long coef_rows(int ns, bool cplx) { return cplx ? 16LL * ((ns + 7) / 8) : coef_ld(ns); }
+
+// Doubles of the coefficients of nk x ns states, and of the bricks' partial sums of one slice of
+// them; an operator application takes both as one scratch, the coefficients first.
+size_t coef_elems(qg_hamiltonian h, int nk, int ns, bool cplx);
+size_t part_elems(qg_hamiltonian h, int nk, int ns, bool cplx);
+// Whether real FP64 states are projected brick by brick (see the rule at its definition).
+bool bricks_for_real(const DevProjectors& pj);
+inline size_t nonlocal_scratch(qg_hamiltonian h, int nk, int ns, bool cplx) {
+    return coef_elems(h, nk, ns, cplx) + (cplx || bricks_for_real(h->pj) ? part_elems(h, nk, ns, cplx) : 0);
+}
+// Kernels brick_project launches for ns real states.
+int brick_project_launches(qg_hamiltonian h, int ns);
+
+// Real: coef[(atom * nch + ch) * coef_ld(ns) + s] = scale[atom * nch + ch] * sum_p P(p) psi_s(p).
+// Complex: coef[((k * ncg + cg) * coef_rows + row) * 4 + c], cg = atom * (nch / 4) + channel group;
+// phase: the tables of ensure_phases (real states: nullptr).
+template <typename T>
+int brick_project(qg_hamiltonian h, int nk, int ns, bool cplx, const T* X, long long ldx, long long ldk,
+                  const double2* phase, const double* scale, double* coef, double* part, cudaStream_t st);
+// HX += sum over spheres and channels conj(P) coef, complex states.
+template <typename T>
+int brick_scatter_z(qg_hamiltonian h, int nk, int ns, T* HX, long long ldx, long long ldk, const double2* phase,
+                    const double* coef, cudaStream_t st);
+
+// Bloch phases exp(i g.r) of nk k-vectors (HOST, 3 each): per k-point nx + ny + nz values of
+// the axes, then one per periodic image; rebuilt when the k-vectors change.
+int ensure_phases(qg_hamiltonian h, int nk, const double* kv, cudaStream_t st, const double2** out);
+
+}  // namespace qg

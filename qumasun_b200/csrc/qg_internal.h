@@ -62,7 +62,28 @@ struct qg_context_s {
 // Frees the context's qg_gram_mixed_d buffers (gram_mixed.cu).
 void qg_release_gram_cache(qg_context c);
 
-// Nonlocal projector tables on the device, in two orders:
+// Nonlocal projector tables by bricks of the grid (nonlocal.cu): the values of every sphere
+// in every block of 8 consecutive x points it meets, and the items, slots and sums that
+// order them.
+struct BrickTables {
+    int nbx = 0, nby = 0, nbricks = 0, nitems = 0, npairs = 0, max_tab = 0, ncg = 0, nimg = 0;
+    int* item_brick = nullptr;
+    int* item_pair = nullptr;
+    int* item_cg = nullptr;
+    int* item_img = nullptr;
+    unsigned long long* wmask = nullptr;
+    int* wtab = nullptr;
+    int* brick_item = nullptr;
+    double* tab = nullptr;
+    int* cg_off = nullptr;   // partial sums of a coefficient group: {2 * pair + half, image}
+    int2* cg_ref = nullptr;
+    int* img = nullptr;      // periodic images, 3 per image
+    DevBuf phase;            // Bloch phases of the k-vectors phase_k (ensure_phases)
+    size_t phase_at = 0;
+    std::vector<double> phase_k;
+};
+
+// Nonlocal projector tables on the device, in two orders and by bricks:
 //  gather side (atom-major): atom a owns points [atom_off[a], atom_off[a+1]) of
 //    pt_g (grid index) and tab[ch*npts + p] (channel values w*Y);
 //  scatter side (grid-point-major): grid point g owns entries
@@ -83,25 +104,7 @@ struct DevProjectors {
     int* ent_atom = nullptr;
     double* ent_val_d = nullptr;
     float* ent_val_f = nullptr;
-    // k-point (complex) side: unwrapped grid coordinates of each point (3 per
-    // point, the image the cube point came from), the point of each scatter
-    // entry, and the Bloch-phase tables for the k-vector zg:
-    //   ztab[ch*npts + p] = tab * cos(theta_p), ztab[(nch + ch)*npts + p] = tab * sin(theta_p),
-    //   zent[(e*nch + ch)*2 + {0,1}] = ent_val * (cos, sin)(theta_p(e)),
-    // theta_p = g . (h * u_p)
-    int* pt_u = nullptr;
-    int* ent_pt = nullptr;
-    double* ztab = nullptr;
-    double* zent = nullptr;
-    std::vector<double> zk;  // k-vectors (3 per k-point) the tables were built for
-    int zcap = 0;            // k-points the table buffers hold
-    bool zready = false;
-    // the same tables in FP32 for complex64 states
-    float* ztab_f = nullptr;
-    float* zent_f = nullptr;
-    std::vector<double> zk_f;
-    int zcap_f = 0;
-    bool zready_f = false;
+    BrickTables bricks;
 };
 
 namespace qg {
@@ -117,7 +120,7 @@ struct qg_hamiltonian_s {
     double* V_d = nullptr;
     float* V_f = nullptr;
     DevProjectors pj;
-    DevBuf coef;      // projector coefficients E*dV*<p|psi>, [ns][na*nch]
+    DevBuf coef;      // projector coefficients E*dV*<p|psi> and the bricks' partial sums
     DevBuf xio, hxio; // staging for the host-buffer entry point
     DevBuf kco;       // per-k-point stencil coefficients of a multi-k apply
     DevBuf scf_work;  // propagation blocks, gradients and inner products (scf.cu)
@@ -240,13 +243,12 @@ inline long long coef_ld(int ns) { return (ns + 15) / 16 * 16; }
 
 // Elements of projector-coefficient scratch ([n_atoms * n_channels][coef_ld(ns)]) one apply of ns states needs.
 size_t coef_scratch_elems(qg_hamiltonian h, int ns);
-// Doubles of complex coefficient scratch ([nk][n_atoms * n_channels][coef_ld(nsk)] {re, im})
-// one k-point apply of nk k-points x nsk states needs.
-size_t coef_scratch_elems_z(qg_hamiltonian h, int nk, int nsk);
 
+// scratch: nonlocal_scratch(h, 1, ns, false) doubles (nonlocal.h), or coef_scratch_elems(h, ns) of
+// T with atom_major, which projects atom by atom straight into the coefficients.
 template <typename T>
 int apply_hamiltonian(qg_hamiltonian h, int ns, const T* X, long long ldx, T* HX, long long ldhx,
-                      T* coef_scratch, cudaStream_t st, PhaseTimer* pt = nullptr);
+                      void* scratch, cudaStream_t st, PhaseTimer* pt = nullptr, bool atom_major = false);
 
 // Inner products dV <p_{a,ch}|psi_s> of ns real states, channel-major like the
 // operator's coefficients: coef[(a * nch + ch) * ldc + s] (hamiltonian.cu).
@@ -254,16 +256,16 @@ int project_inner_d(qg_hamiltonian h, int ns, const double* X, long long ldx, do
                     cudaStream_t st);
 
 // Complex k-point H (kpoint.cu): state s has its real part at X + s*ldx and its
-// imaginary part N elements later; coef_scratch holds 2*coef_scratch_elems(h, ns) doubles.
+// imaginary part N elements later; scratch holds nonlocal_scratch(h, 1, ns, true) doubles.
 template <typename T>
 int apply_hamiltonian_z(qg_hamiltonian h, int ns, const T* X, long long ldx, T* HX, long long ldhx,
-                        T* coef_scratch, cudaStream_t st, PhaseTimer* pt = nullptr);
+                        double* scratch, cudaStream_t st, PhaseTimer* pt = nullptr);
 // Several k-points in one pass: nk k-vectors kv (3 each, bohr^-1), nsk states per k-point,
-// state s of k-point k at X + k*ldk + s*ldx (HX + k*ldkh + s*ldhx); coef_scratch holds
-// 2*coef_scratch_elems(h, nk*nsk) doubles.
+// state s of k-point k at X + k*ldk + s*ldx (HX + k*ldkh + s*ldhx); scratch holds
+// nonlocal_scratch(h, nk, nsk, true) doubles.
 template <typename T>
 int apply_hamiltonian_zk(qg_hamiltonian h, int nk, const double* kv, int nsk, const T* X, long long ldx,
-                         long long ldk, T* HX, long long ldhx, long long ldkh, T* coef_scratch, cudaStream_t st,
+                         long long ldk, T* HX, long long ldhx, long long ldkh, double* scratch, cudaStream_t st,
                          PhaseTimer* pt = nullptr);
 
 }  // namespace qg

@@ -17,6 +17,7 @@
 #include <cmath>
 #include <vector>
 
+#include "nonlocal.h"
 #include "qg_internal.h"
 
 namespace qg {
@@ -439,11 +440,8 @@ int qg_td_taylor4_z(qg_hamiltonian h, int ns, double dt, double* X, long long ld
     QG_TRY(h->scf_work.reserve((size_t)2 * ns * ldw * sizeof(double)));
     double* W1 = h->scf_work.as<double>();
     double* W2 = W1 + (size_t)ns * ldw;
-    double* coef = nullptr;
-    if (h->pj.na > 0) {
-        QG_TRY(h->coef.reserve(qg::coef_scratch_elems_z(h, 1, ns) * sizeof(double)));
-        coef = h->coef.as<double>();
-    }
+    QG_TRY(h->coef.reserve(qg::nonlocal_scratch(h, 1, ns, true) * sizeof(double)));
+    double* coef = h->coef.as<double>();
     const int g = qg::grid_for((long long)ns * N);
     const double c2 = dt * dt / 2.0;
     const double c3 = c2 * dt / 3.0;

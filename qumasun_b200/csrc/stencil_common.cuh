@@ -17,13 +17,6 @@ struct HamArgs {
     int zslab;
     T c0;
     T cx[4], cy[4], cz[4];
-    // nonlocal scatter side (row == nullptr: no nonlocal term)
-    const int* row;
-    const int* ent_atom;
-    const T* ent_val;
-    int nch;
-    long long ldc;   // coefficient row length (states, padded to 16)
-    const T* coef;   // [na * nch][ldc]
     int* err;        // device status word: nonzero after a bounded wait gave up
     int stall;       // test hook: the ring kernels' producer issues nothing, so the
                      // consumers' bounded waits run out (QG_ERR_TIMEOUT)

@@ -353,7 +353,6 @@ bool stencil_pair_ok(const HamArgs<T>& a, int order) {
     constexpr int PX = 16 / sizeof(T);
     const int R = order == 2 ? 1 : (order == 8 ? 4 : 3);
     if (order != 2 && order != 4 && order != 6 && order != 8) return false;
-    if (a.row) return false;
     if (a.nsk > 0) return false;
     if (a.nx % PX != 0 || ((uintptr_t)a.X % 16) || ((uintptr_t)a.HX % 16) || ((uintptr_t)a.V % 16) ||
         (a.ldx % PX) || (a.ldhx % PX) || !a.err || a.ny < 2 * R || a.nx < 2 * R || a.nz < 2 * R)

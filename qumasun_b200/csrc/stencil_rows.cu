@@ -365,7 +365,7 @@ bool stencil_rows_ok(const HamArgs<T>& a, int order, bool vring) {
     constexpr int PX = 16 / sizeof(T);
     if (order != 2 && order != 4 && order != 6 && order != 8) return false;
     const int R = order == 2 ? 1 : (order == 8 ? 4 : 3);
-    if (a.row || a.nsk > 0) return false;
+    if (a.nsk > 0) return false;
     if (a.nx % PX != 0 || ((uintptr_t)a.X % 16) || ((uintptr_t)a.HX % 16) || ((uintptr_t)a.V % 16) ||
         (a.ldx % PX) || (a.ldhx % PX) || !a.err || a.ny < 2 * R || a.nx < 2 * R || a.nz < 2 * R)
         return false;

@@ -542,7 +542,6 @@ bool stencil_tma_ok(const HamArgs<T>& a, int order, int nc) {
     const int R = order == 2 ? 1 : (order == 8 ? 4 : 3);
     if (nc != 1 && nc != 2) return false;
     if (nc == 2 && ((order != 2 && order != 6 && order != 8) || (a.xim % PX) || (a.hxim % PX))) return false;
-    if (a.row) return false;  // the nonlocal scatter runs in k_scatter_all on this path
     if (a.nx % PX != 0 || ((uintptr_t)a.X % 16) || ((uintptr_t)a.HX % 16) || ((uintptr_t)a.V % 16) ||
         (a.ldx % PX) || (a.ldhx % PX) || !a.err || a.ny < 2 * R || a.nx < 2 * R)
         return false;

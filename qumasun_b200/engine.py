@@ -731,8 +731,8 @@ class Hamiltonian:
         check(lib().qg_hamiltonian_set_stencil_kernel(self.h, v), "qg_hamiltonian_set_stencil_kernel")
 
     def set_nonlocal_blocking(self, project_states=0, scatter_states=0, project_parts=0):
-        """States per projection block (1/2/4/8/16), per scatter group (4/8) and blocks per
-        atom in the projection (1-8); 0 = engine's choice."""
+        """Real states: states per projection block (1/2/4/8/16), per scatter group (4/8) and
+        blocks per atom in the projection (1-8); 0 = engine's choice."""
         check(lib().qg_hamiltonian_set_nonlocal_blocking(self.h, project_states, scatter_states, project_parts),
               "qg_hamiltonian_set_nonlocal_blocking")
 

@@ -1,0 +1,121 @@
+"""Nonlocal projectors through brick tables (cells of more than 16 atoms, every k-point
+state) against the CPU oracle, at the edges of the bricks (16 x 8 x 4 points: rows that are no
+multiple of 8 or 16, odd rows, layers that end inside a brick, spheres that wrap), of the state
+tiles (8 states per warp, 64 per block) and of the row strides and alignments that the
+vector loads have to leave to the scalar ones.
+
+Tolerance: a projector sum has at most a few thousand terms in FP64, added pairwise over
+bricks: well below 1e-12 of the state's norm, the bound of the other operator tests. The
+nonlocal part alone (H x minus the local part, ~1e-3 of the total) is held to 1e-10 of its own size."""
+import numpy as np
+import pytest
+
+import oracle as O
+from qumasun_b200.cell import build_cell, initial_states
+
+pytestmark = pytest.mark.gpu
+CELLS = {
+    "multiple": dict(reps=(1, 1, 3), grid=(16, 16, 48)),
+    "ragged": dict(reps=(1, 1, 3), grid=(20, 18, 50), displacement=0.1, seed=3),
+    "odd": dict(reps=(3, 1, 1), grid=(45, 17, 15), displacement=0.1, seed=4),
+    "wrap": dict(reps=(1, 3, 1), grid=(12, 34, 10), a0=4.4),
+}
+
+
+def rel(a, b):
+    return (np.linalg.norm(a - b, axis=-1) / np.linalg.norm(b, axis=-1)).max()
+
+
+def padded(X, pad, shift):
+    """X as a strided view: rows `pad` elements longer, first element `shift` elements in."""
+    import torch
+    ns, n = X.shape
+    buf = torch.full((ns * (n + pad) + shift,), float("nan"), dtype=X.dtype, device="cuda")
+    view = buf[shift:].view(ns, n + pad)[:, :n]
+    view.copy_(X)
+    return buf, view
+
+
+@pytest.mark.parametrize("ns", [1, 7, 8, 9, 65])
+@pytest.mark.parametrize("name", sorted(CELLS))
+def test_real_projection_matches_oracle(cuda_ctx, name, ns):
+    import torch
+    from qumasun_b200 import Hamiltonian
+    cell = build_cell(**CELLS[name])
+    X = initial_states(ns, cell.N, seed=ns)
+    H = Hamiltonian(cuda_ctx, cell)
+    Xd = torch.from_numpy(X).cuda()
+    out = H.apply(Xd)
+    ref = O.hamiltonian_apply(cell, X)
+    loc = O.hamiltonian_kpoint_local(cell, (0.0, 0.0, 0.0), np.concatenate([X, 0 * X], 1))[:, :cell.N]
+    got = out.cpu().numpy()
+    assert rel(got, ref) < 1e-12 and rel(got - loc, ref - loc) < 1e-10
+    # the atom-by-atom kernel, and a state's bits whatever its batch
+    H.set_nonlocal_blocking(0, 0, 1)
+    assert rel(H.apply(Xd).cpu().numpy(), ref) < 1e-12
+    H.set_nonlocal_blocking(0, 0, 0)
+    if ns > 1:
+        assert torch.equal(H.apply(Xd[ns - 1:]), out[ns - 1:])
+    # rows of an odd length that start on 8 bytes
+    for pad, shift in ((1, 1), (2, 0), (0, 1)):
+        xb, xv = padded(Xd, pad, shift)
+        hb, hv = padded(torch.zeros_like(Xd), pad, shift)
+        torch.cuda.synchronize()
+        H.apply_device(ns, xv.data_ptr(), hv.data_ptr(), cell.N + pad, cell.N + pad)
+        cuda_ctx.synchronize()
+        assert rel(hv.cpu().numpy(), got) < 1e-14, (pad, shift)  # another stencil kernel may run
+        del xb, hb
+    H.close()
+
+
+@pytest.mark.parametrize("dtype", ["complex128", "complex64"])
+@pytest.mark.parametrize("ns", [1, 5, 33])
+@pytest.mark.parametrize("name", sorted(CELLS))
+def test_kpoint_projection_and_scatter_match_oracle(cuda_ctx, name, ns, dtype):
+    import ctypes as C
+    import torch
+    from qumasun_b200 import Hamiltonian
+    from qumasun_b200.engine import lib
+    f64 = dtype == "complex128"
+    cell = build_cell(**CELLS[name])
+    n2 = 2 * cell.N
+    kv = np.array([[0.11, -0.23, 0.31], [0.0, 0.0, 0.0], [-0.3, 0.07, 0.02]])
+    X = initial_states(3 * ns, n2, seed=ns).reshape(3, ns, n2)
+    Xd = torch.from_numpy(X).cuda().to(torch.float64 if f64 else torch.float32)
+    H = Hamiltonian(cuda_ctx, cell)
+    many = H.apply_zk(kv, Xd)
+    for k in range(3):
+        ref = O.hamiltonian_kpoint_apply(cell, tuple(kv[k]), X[k])
+        loc = O.hamiltonian_kpoint_local(cell, tuple(kv[k]), X[k])
+        got = many[k].double().cpu().numpy()
+        # FP32 states carry 2^-24 of rounding per stencil term: the bound of the complex64 tests
+        assert rel(got, ref) < (1e-12 if f64 else 2e-6), k
+        if f64:
+            assert rel(got - loc, ref - loc) < 1e-10, k
+    H.set_kvector(kv[2])
+    assert torch.equal(H.apply_z(Xd[2]), many[2])
+    fn = lib().qg_hamiltonian_apply_z if f64 else lib().qg_hamiltonian_apply_zf
+    for pad, shift in ((1, 1), (2, 0), (0, 1)):
+        xb, xv = padded(Xd[2], pad, shift)
+        hb, hv = padded(torch.zeros_like(Xd[2]), pad, shift)
+        torch.cuda.synchronize()
+        assert fn(H.h, ns, C.c_void_p(xv.data_ptr()), n2 + pad, C.c_void_p(hv.data_ptr()), n2 + pad) == 0
+        cuda_ctx.synchronize()
+        assert rel(hv.double().cpu().numpy(), many[2].double().cpu().numpy()) < (1e-14 if f64 else 1e-6), (pad, shift)
+        del xb, hb
+    H.close()
+
+
+@pytest.mark.parametrize("kw", [dict(grid=(13, 11, 9)), dict(grid=(27, 17, 15), displacement=0.05, seed=1)],
+                         ids=["8-atoms-tiny", "8-atoms"])
+@pytest.mark.parametrize("f64", [True, False], ids=["f64", "f32"])
+def test_odd_grid_split_scatter_matches_oracle(cuda_ctx, kw, f64):
+    """Odd rows: stencil and scatter are two kernels."""
+    import torch
+    from qumasun_b200 import Hamiltonian
+    cell = build_cell(**kw)
+    X = initial_states(9, cell.N, seed=2)
+    H = Hamiltonian(cuda_ctx, cell)
+    got = H.apply(torch.from_numpy(X).cuda().to(torch.float64 if f64 else torch.float32)).double().cpu().numpy()
+    H.close()
+    assert rel(got, O.hamiltonian_apply(cell, X)) < (1e-12 if f64 else 2e-6)
