@@ -408,14 +408,13 @@ static int launch_project_nch(const DevProjectors& pj, const T* tab, int ns, con
     return QG_OK;
 }
 
-// scale[atom * nch + ch] multiplies each sum (nullptr: E_k * dV, the operator's coefficients).
 template <typename T>
 static int launch_project(const DevProjectors& pj, int ns, const T* X, long long ldx, T* coef, long long ldc,
-                          int forced_sb, int forced_parts, cudaStream_t st, const double* scale = nullptr) {
+                          int forced_sb, int forced_parts, cudaStream_t st) {
     const T* tab;
     if constexpr (sizeof(T) == 8) tab = reinterpret_cast<const T*>(pj.tab_d);
     else tab = reinterpret_cast<const T*>(pj.tab_f);
-    if (!scale) scale = pj.ch_scale;
+    const double* scale = pj.ch_scale;
     const int parts = project_parts(pj, forced_parts);
     const int sb = pick_project_sb(pj.na * parts, ns, forced_sb);
     switch (pj.nch) {
@@ -424,11 +423,6 @@ static int launch_project(const DevProjectors& pj, int ns, const T* X, long long
         case 16: return launch_project_nch<T, 16>(pj, tab, ns, X, ldx, coef, ldc, sb, parts, st, scale);
         default: return QG_ERR_UNSUPPORTED;
     }
-}
-
-int project_inner_d(qg_hamiltonian h, int ns, const double* X, long long ldx, double* coef, long long ldc,
-                    cudaStream_t st) {
-    return launch_project<double>(h->pj, ns, X, ldx, coef, ldc, h->proj_sb, h->proj_parts, st, h->pj.ch_dv);
 }
 
 // 16-byte vector of T (the unit the scatter reads the coefficients in).

@@ -250,11 +250,6 @@ template <typename T>
 int apply_hamiltonian(qg_hamiltonian h, int ns, const T* X, long long ldx, T* HX, long long ldhx,
                       void* scratch, cudaStream_t st, PhaseTimer* pt = nullptr, bool atom_major = false);
 
-// Inner products dV <p_{a,ch}|psi_s> of ns real states, channel-major like the
-// operator's coefficients: coef[(a * nch + ch) * ldc + s] (hamiltonian.cu).
-int project_inner_d(qg_hamiltonian h, int ns, const double* X, long long ldx, double* coef, long long ldc,
-                    cudaStream_t st);
-
 // Complex k-point H (kpoint.cu): state s has its real part at X + s*ldx and its
 // imaginary part N elements later; scratch holds nonlocal_scratch(h, 1, ns, true) doubles.
 template <typename T>

@@ -19,6 +19,7 @@
 
 #include "nonlocal.h"
 #include "qg_internal.h"
+#include "stencil_common.cuh"
 
 namespace qg {
 namespace {
@@ -219,86 +220,91 @@ __global__ void __launch_bounds__(kThreads) k_td_update(int ns, long long N, dou
 
 // ---------------------------------------------------------------- nonlocal forces
 
-// out_d[c][i] = coef_c * d psi_c / d axis at i, 8th order, periodic; cf[c*12 + 4*axis + (0..3)]
-// holds (c1, c2, c3, c4) * coef_c / (840 h) with (672, -168, 32, -3), summed from the
-// outermost pair inwards as Gradient8th_{x,y,z}_halo_f (GridGradient8th.h:19-190) does.
+// out_d[c][i] = d psi_c / d axis at i, 8th order, periodic, any shape; (672, -168, 32, -3) s_axis with
+// s = 1 / (840 h), summed from the outermost pair inwards as Gradient8th_{x,y,z}_halo_f
+// (GridGradient8th.h:19-190) does.
 __global__ void __launch_bounds__(kThreads) k_gradient8(int nx, int ny, int nz, int nc, const double* __restrict__ X,
-                                                        long long ldx, const int* __restrict__ sidx,
-                                                        const double* __restrict__ cf, double* __restrict__ out,
-                                                        long long ldo) {
+                                                        long long ldx, const int* __restrict__ sidx, double sx,
+                                                        double sy, double sz, double* __restrict__ out, long long ldo) {
     const long long N = (long long)nx * ny * nz;
     const long long total = (long long)nc * N;
+    const double sc[3] = {sx, sy, sz};
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
         const int c = (int)(t / N);
         const long long i = t - (long long)c * N;
         const int ix = (int)(i % nx), iy = (int)((i / nx) % ny), iz = (int)(i / ((long long)nx * ny));
         const double* p = X + (long long)sidx[c] * ldx;
-        const double* k = cf + c * 12;
         double g[3];
 #pragma unroll
         for (int ax = 0; ax < 3; ++ax) {
+            const int at = ax == 0 ? ix : (ax == 1 ? iy : iz), n = ax == 0 ? nx : (ax == 1 ? ny : nz);
+            const long long step = ax == 0 ? 1 : (ax == 1 ? nx : (long long)nx * ny);
             double d[5];  // p(+s) - p(-s), s = 1..4
 #pragma unroll
-            for (int s = 1; s <= 4; ++s) {
-                long long ip, im;
-                if (ax == 0) {
-                    ip = i - ix + (ix + s) % nx;
-                    im = i - ix + (ix - s + nx) % nx;
-                } else if (ax == 1) {
-                    ip = i + (long long)(((iy + s) % ny) - iy) * nx;
-                    im = i + (long long)(((iy - s + ny) % ny) - iy) * nx;
-                } else {
-                    ip = i + (long long)(((iz + s) % nz) - iz) * nx * ny;
-                    im = i + (long long)(((iz - s + nz) % nz) - iz) * nx * ny;
-                }
-                d[s] = p[ip] - p[im];
-            }
-            g[ax] = k[4 * ax + 3] * d[4] + k[4 * ax + 2] * d[3] + k[4 * ax + 1] * d[2] + k[4 * ax + 0] * d[1];
+            for (int s = 1; s <= 4; ++s) d[s] = p[i + ((at + s) % n - at) * step] - p[i + ((at - s + 4 * n) % n - at) * step];
+            g[ax] = (-3.0 * d[4] + 32.0 * d[3] - 168.0 * d[2] + 672.0 * d[1]) * sc[ax];
         }
-        out[(long long)c * ldo + i] = g[0];
-        out[(long long)(nc + c) * ldo + i] = g[1];
-        out[(long long)(2 * nc + c) * ldo + i] = g[2];
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) out[(long long)(ax * nc + c) * ldo + i] = g[ax];
     }
 }
 
-// Per chunk of nc states: e[c] = sum_{a,ch} E inner^2 and, for every atom,
-// f[3a + d] += sum_c sum_ch E inner dinner_d (states in order, channels in order).
-__global__ void __launch_bounds__(kThreads) k_force_reduce(int na, int nch, int nc, long long ldc,
-                                                           const double* __restrict__ inner,
-                                                           const double* __restrict__ dinner,  // [3][na*nch][ldc]
-                                                           const double* __restrict__ chE, const int* __restrict__ use,
-                                                           double* __restrict__ forces, double* __restrict__ e_out) {
-    const long long plane = (long long)na * nch * ldc;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < na + nc; t += gridDim.x * blockDim.x) {
-        if (t < na) {
-            const int a = t;
-            double f[3] = {forces[3 * a], forces[3 * a + 1], forces[3 * a + 2]};
-            for (int c = 0; c < nc; ++c) {
-                if (!use[c]) continue;
-                double fi[3] = {0.0, 0.0, 0.0};
-                for (int ch = 0; ch < nch; ++ch) {
-                    const long long q = (long long)(a * nch + ch) * ldc + c;
-                    const double E = chE[a * nch + ch];
-                    const double in = inner[q];
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) fi[d] += dinner[d * plane + q] * in * E;
-                }
-#pragma unroll
-                for (int d = 0; d < 3; ++d) f[d] += fi[d];
-            }
-            forces[3 * a] = f[0];
-            forces[3 * a + 1] = f[1];
-            forces[3 * a + 2] = f[2];
-        } else {
-            const int c = t - na;
-            double e = 0.0;
-            for (int q = 0; q < na * nch; ++q) {
-                const double in = inner[(long long)q * ldc + c];
-                e += in * in * chE[q];
-            }
-            e_out[c] = e;
+// Energies: e[s] = sum_q E_q inner[q][s]^2 over the channels of all atoms, 32 states per block; each
+// warp adds a contiguous eighth of the channels, the eighths are added in order.
+__global__ void __launch_bounds__(kThreads) k_nonlocal_energy(int nq, int ns, long long rows,
+                                                              const double* __restrict__ inner,
+                                                              const double* __restrict__ chE, double* __restrict__ e) {
+    __shared__ double sm[8][32];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, s = blockIdx.x * 32 + lane;
+    double v = 0.0;
+    if (s < ns) {
+#pragma unroll 4
+        for (int q = nq * w / 8; q < nq * (w + 1) / 8; ++q) {
+            const double in = inner[(long long)q * rows + s];
+            v += in * in * __ldg(&chE[q]);
         }
     }
+    sm[w][lane] = v;
+    __syncthreads();
+    if (w == 0 && s < ns) {
+        v = sm[0][lane];
+#pragma unroll
+        for (int i = 1; i < 8; ++i) v += sm[i][lane];
+        e[s] = v;
+    }
+}
+
+// Forces of one atom per block: forces[3a + d] += sum_s -2 occ_s sum_ch E inner_s dinner_{d,s} over nc
+// states, idx their rows of inner, occ their occupations, rows d * nc + c of dinner. A thread takes
+// states blockDim apart, the threads are added in a fixed tree.
+__global__ void __launch_bounds__(kThreads) k_force_reduce(int nch, int nc, const int* __restrict__ idx,
+                                                           const double* __restrict__ occ, long long rows,
+                                                           const double* __restrict__ inner, long long drows,
+                                                           const double* __restrict__ dinner,
+                                                           const double* __restrict__ chE, double* __restrict__ forces) {
+    __shared__ double sm[3][kThreads];
+    double f[3] = {0.0, 0.0, 0.0};
+    for (int c = threadIdx.x; c < nc; c += kThreads) {
+        double fi[3] = {0.0, 0.0, 0.0};
+        for (int ch = 0; ch < nch; ++ch) {
+            const long long q = (long long)blockIdx.x * nch + ch;
+            const double in = inner[q * rows + idx[c]] * __ldg(&chE[q]);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) fi[d] += in * dinner[q * drows + d * nc + c];
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) f[d] += -2.0 * occ[c] * fi[d];
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) sm[d][threadIdx.x] = f[d];
+    __syncthreads();
+    for (int o = kThreads / 2; o > 0; o >>= 1) {
+        if (threadIdx.x < o)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) sm[d][threadIdx.x] += sm[d][threadIdx.x + o];
+        __syncthreads();
+    }
+    if (threadIdx.x < 3) forces[3 * blockIdx.x + threadIdx.x] += sm[threadIdx.x][0];
 }
 
 }  // namespace
@@ -476,61 +482,59 @@ int qg_nonlocal_force_d(qg_hamiltonian h, int ns, const double* X, long long ldx
     }
     QG_CUDA_TRY(cudaSetDevice(h->ctx->device));
     cudaStream_t st = h->ctx->stream;
-    // chunk of states whose three gradients fit ~1 GiB
-    const int nc_max = (int)std::max<long long>(1, std::min<long long>(ns, (1LL << 30) / (3 * N * 8)));
-    const long long ldc = qg::coef_ld(nc_max);
-    const size_t grad_elems = (size_t)3 * nc_max * N;
-    const size_t inner_elems = (size_t)4 * na * nch * ldc;
-    const size_t meta = (size_t)nc_max * (12 + 1) + 3 * (size_t)na + nc_max;  // coefficients, flags, forces, energies
-    QG_TRY(h->scf_work.reserve((grad_elems + inner_elems + meta) * sizeof(double) + (size_t)2 * nc_max * sizeof(int)));
+    // the inner products of all states, then chunk by chunk the occupied states' gradients and
+    // their inner products (three gradients of a chunk fit ~1 GiB)
+    std::vector<int> used;
+    std::vector<double> f;
+    for (int s = 0; s < ns; ++s)
+        if (occ[s] > 0.0) {
+            used.push_back(s);
+            f.push_back(occ[s]);
+        }
+    const int nu = (int)used.size();
+    const int nc_max = (int)std::max<long long>(1, std::min<long long>(nu, (1LL << 30) / (3 * N * 8)));
+    const size_t ce = qg::coef_elems(h, 1, ns, false), de = qg::coef_elems(h, 1, 3 * nc_max, false);
+    const size_t pe = std::max(qg::part_elems(h, 1, ns, false), qg::part_elems(h, 1, 3 * nc_max, false));
+    const size_t grad_elems = nu > 0 ? ((size_t)3 * nc_max * N + 1) / 2 * 2 : 0;  // what follows stays 16-byte aligned
+    QG_TRY(h->scf_work.reserve((grad_elems + ce + de + pe + 3 * (size_t)na + ns + 2 * (size_t)nu) * sizeof(double)));
     double* grad = h->scf_work.as<double>();
     double* inner = grad + grad_elems;
-    double* dinner = inner + (size_t)na * nch * ldc;
-    double* cf = inner + inner_elems;
-    double* fdev = cf + (size_t)nc_max * 12;
+    double* dinner = inner + ce;
+    double* part = dinner + de;
+    double* fdev = part + pe;       // forces, then the energies: one copy back
     double* edev = fdev + 3 * (size_t)na;
-    int* sidx = reinterpret_cast<int*>(edev + nc_max);
-    int* use = sidx + nc_max;
+    double* odev = edev + ns;
+    int* sidx = reinterpret_cast<int*>(odev + nu);
     QG_CUDA_TRY(cudaMemcpyAsync(fdev, forces, 3 * (size_t)na * sizeof(double), cudaMemcpyHostToDevice, st));
-    const double h3[3] = {h->hx, h->hy, h->hz};
-    const double kk[4] = {672.0, -168.0, 32.0, -3.0};
-    double ev = 0.0;
-    std::vector<double> e_chunk(nc_max), cf_h((size_t)nc_max * 12);
-    std::vector<int> sidx_h(nc_max), use_h(nc_max);
-    for (int s0 = 0; s0 < ns; s0 += nc_max) {
-        const int nc = std::min(nc_max, ns - s0);
-        for (int c = 0; c < nc; ++c) {
-            const double o = occ[s0 + c];
-            const double coef = o > 0.0 ? -2.0 * o : 1.0;  // energies of unoccupied states too
-            sidx_h[c] = s0 + c;
-            use_h[c] = o > 0.0;
-            for (int ax = 0; ax < 3; ++ax)
-                for (int j = 0; j < 4; ++j) cf_h[(size_t)c * 12 + 4 * ax + j] = kk[j] * coef / (840.0 * h3[ax]);
-        }
-        QG_CUDA_TRY(cudaMemcpyAsync(cf, cf_h.data(), (size_t)nc * 12 * sizeof(double), cudaMemcpyHostToDevice, st));
-        QG_CUDA_TRY(cudaMemcpyAsync(sidx, sidx_h.data(), nc * sizeof(int), cudaMemcpyHostToDevice, st));
-        QG_CUDA_TRY(cudaMemcpyAsync(use, use_h.data(), nc * sizeof(int), cudaMemcpyHostToDevice, st));
-        qg::k_gradient8<<<qg::grid_for((long long)nc * N), qg::kThreads, 0, st>>>(h->nx, h->ny, h->nz, nc, X, ldx, sidx,
-                                                                                 cf, grad, N);
-        QG_TRY(qg::project_inner_d(h, nc, X + (long long)s0 * ldx, ldx, inner, ldc, st));
-        for (int d = 0; d < 3; ++d)
-            QG_TRY(qg::project_inner_d(h, nc, grad + (size_t)d * nc * N, N, dinner + (size_t)d * na * nch * ldc, ldc,
-                                       st));
-        qg::k_force_reduce<<<(na + nc + qg::kThreads - 1) / qg::kThreads, qg::kThreads, 0, st>>>(
-            na, nch, nc, ldc, inner, dinner, h->pj.ch_E, use, fdev, edev);
-        QG_CUDA_TRY(cudaGetLastError());
-        QG_CUDA_TRY(cudaMemcpyAsync(e_chunk.data(), edev, nc * sizeof(double), cudaMemcpyDeviceToHost, st));
-        QG_CUDA_TRY(cudaStreamSynchronize(st));
-        for (int c = 0; c < nc; ++c) {
-            // the unoccupied states' gradients were formed with coef 1: their energy is
-            // still E inner^2, they add no force (use = 0) and nothing to EV
-            if (e_state) e_state[s0 + c] = e_chunk[c];
-            if (use_h[c]) ev += e_chunk[c] * occ[s0 + c];
-        }
+    if (nu > 0) {
+        QG_CUDA_TRY(cudaMemcpyAsync(odev, f.data(), nu * sizeof(double), cudaMemcpyHostToDevice, st));
+        QG_CUDA_TRY(cudaMemcpyAsync(sidx, used.data(), nu * sizeof(int), cudaMemcpyHostToDevice, st));
     }
-    QG_CUDA_TRY(cudaMemcpyAsync(forces, fdev, 3 * (size_t)na * sizeof(double), cudaMemcpyDeviceToHost, st));
+    const double h3[3] = {h->hx, h->hy, h->hz};
+    QG_TRY(qg::brick_project<double>(h, 1, ns, false, X, ldx, 0, nullptr, h->pj.ch_dv, inner, part, st));
+    qg::k_nonlocal_energy<<<(ns + 31) / 32, qg::kThreads, 0, st>>>(na * nch, ns, qg::coef_rows(ns, false), inner, h->pj.ch_E,
+                                                                 edev);
+    for (int s0 = 0; s0 < nu; s0 += nc_max) {
+        const int nc = std::min(nc_max, nu - s0);
+        const int rc = qg::launch_gradient8(X, ldx, ns, sidx + s0, nc, grad, h->nx, h->ny, h->nz, h3, h->ctx->dev_status, st);
+        if (rc == QG_ERR_UNSUPPORTED)  // odd rows: any shape
+            qg::k_gradient8<<<qg::grid_for((long long)nc * N), qg::kThreads, 0, st>>>(
+                h->nx, h->ny, h->nz, nc, X, ldx, sidx + s0, 1.0 / (840.0 * h3[0]), 1.0 / (840.0 * h3[1]),
+                1.0 / (840.0 * h3[2]), grad, N);
+        else QG_TRY(rc);
+        QG_TRY(qg::brick_project<double>(h, 1, 3 * nc, false, grad, N, 0, nullptr, h->pj.ch_dv, dinner, part, st));
+        qg::k_force_reduce<<<na, qg::kThreads, 0, st>>>(nch, nc, sidx + s0, odev + s0, qg::coef_rows(ns, false), inner,
+                                                        qg::coef_rows(3 * nc, false), dinner, h->pj.ch_E, fdev);
+    }
+    QG_CUDA_TRY(cudaGetLastError());
+    std::vector<double> back(3 * (size_t)na + ns);
+    QG_CUDA_TRY(cudaMemcpyAsync(back.data(), fdev, back.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     QG_CUDA_TRY(cudaStreamSynchronize(st));
-    if (ev_sum) *ev_sum = ev;
+    std::copy_n(back.data(), 3 * (size_t)na, forces);
+    const double* e = back.data() + 3 * (size_t)na;
+    if (e_state) std::copy_n(e, ns, e_state);
+    if (ev_sum)
+        for (int i = 0; i < nu; ++i) *ev_sum += e[used[i]] * f[i];
     return QG_OK;
 }
 
