@@ -12,12 +12,12 @@
 //   k_conv_fwd     out[co][v] = b[co] + sum_ci sum_tap W[co][ci][tap] in[ci][v + off(tap)];
 //                  the input tile (+ 1-voxel periodic halo) of one channel and that
 //                  channel's weights, stored [tap][co], sit in shared memory;
-//   backward data  the same kernel with the weights transposed and the taps flipped
-//                  (transposed convolution = convolution on a periodic grid), times
-//                  the ReLU mask of the layer below;
-//   k_conv_wgrad   dW[co][ci][tap] = sum_v dout[co][v] in[ci][v + off(tap)] per tile,
-//                  one thread per (ci, tap) holding all co, tile partials summed in a
-//                  fixed order (deterministic);
+// Backward pass on the tensor cores, FP32 gradients as three BF16 pieces (described below):
+//   k_dgrad_mma    backward data of the 16 -> 16 layers (transposed convolution = convolution
+//                  with transposed weights and flipped taps on a periodic grid) times the ReLU
+//                  mask of the layer below; the 1 -> 16 step runs in k_conv_fwd;
+//   k_wgrad_mma    dW[co][ci][tap] = sum_v dout[co][v] in[ci][v + off(tap)], tiles in turn per
+//                  block, the blocks' sums added in a fixed order (deterministic);
 //   k_adam         Adam on FP32 master weights, BF16 copies for the kernels.
 // Forward pass on the tensor cores (the default where nx is a multiple of 8):
 //   k_conv_tc      every layer as 27 tcgen05.mma per z plane over shared-memory halo
@@ -54,6 +54,11 @@ struct Grid {
 };
 
 __device__ __forceinline__ int wrapi(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
+
+__device__ __forceinline__ int wrap_any(int i, int n) {
+    i %= n;
+    return i < 0 ? i + n : i;
+}
 
 __device__ __forceinline__ float ldf(const __nv_bfloat16* p) { return __bfloat162float(*p); }
 __device__ __forceinline__ float ldf(const float* p) { return *p; }
@@ -122,75 +127,244 @@ __global__ void __launch_bounds__(TV) k_conv_fwd(const TI* __restrict__ in, cons
     }
 }
 
-// Partial weight/bias gradients of one tile: part[blk][co][ci*27 + tap] and part[blk][COUT*CIN*27 + co].
-// Thread k < CIN*27 handles (ci, tap) for all co; bias by threads k < COUT.
-template <int CIN, int COUT, typename TI>
-__global__ void __launch_bounds__(448) k_conv_wgrad(const TI* __restrict__ in, const float* __restrict__ dout,
-                                                    float* __restrict__ part, Grid g) {
-    __shared__ __nv_bfloat16 tin[CIN * HV];  // the layer inputs are bf16 activations
-    __shared__ __align__(16) float dt[TV * COUT];  // [voxel][co]
-    const int tile = blockIdx.x, b = blockIdx.y;
-    const int bx = (tile % g.tx) * TX, by = ((tile / g.tx) % g.ty) * TY, bz = (tile / (g.tx * g.ty)) * TZ;
-    const int t = threadIdx.x;
-    const TI* inb = in + (long long)b * CIN * g.N;
-    for (int i = t; i < CIN * HV; i += blockDim.x) {
-        const int ci = i / HV, h = i % HV;
-        const int hx = h % HX, hy = (h / HX) % HY, hz = h / (HX * HY);
-        const int gx = wrapi(bx + hx - 1, g.nx), gy = wrapi(by + hy - 1, g.ny), gz = wrapi(bz + hz - 1, g.nz);
-        tin[i] = __float2bfloat16(ldf(inb + (long long)ci * g.N + gx + (long long)g.nx * (gy + (long long)g.ny * gz)));
+// ---------------- backward pass on the tensor cores (mma.sync m16n8k16, BF16 in, FP32 sums)
+// The FP32 gradients enter as three BF16 pieces (d = d1 + d2 + d3 to 2^-24), the activations and
+// weights are BF16 already, so the products are those of the FP32 kernels; the FP32 sums of a
+// tile are added to the running sums with ordinary rounding. Bound: shared-memory reads of the
+// operands (ldmatrix); one layer of 16 x 16 channels at 32 states of 40^3 is 14 G multiply-adds.
+// Operand tiles are [voxel][16 channels], 32 bytes a voxel; the two 16-byte halves of a voxel
+// change places every 4 voxels, so the 8 rows of any ldmatrix fall into different banks.
+__device__ __forceinline__ int half_at(int v, int h) { return (2 * v + (h ^ ((v >> 2) & 1))) * 8; }  // in elements
+
+__device__ __forceinline__ void ldm4(uint32_t (&r)[4], const __nv_bfloat16* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldm4t(uint32_t (&r)[4], const __nv_bfloat16* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// 8 channels of one voxel as three BF16 pieces into the half h of voxel v of each piece's tile.
+__device__ __forceinline__ void put_pieces(__nv_bfloat16* tile, int piece_elems, int v, int h, const float (&d)[8]) {
+    __align__(16) __nv_bfloat16 p[3][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        p[0][i] = __float2bfloat16(d[i]);
+        const float r1 = d[i] - __bfloat162float(p[0][i]);
+        p[1][i] = __float2bfloat16(r1);
+        p[2][i] = __float2bfloat16(r1 - __bfloat162float(p[1][i]));
     }
-    for (int i = t; i < TV * COUT; i += blockDim.x) {
-        const int vx = i / COUT, co = i % COUT;
-        const int lx = vx % TX, ly = (vx / TX) % TY, lz = vx / (TX * TY);
-        const int x = bx + lx, y = by + ly, z = bz + lz;
-        float d = 0.f;  // voxels outside the grid (partial tiles) contribute nothing
-        if (x < g.nx && y < g.ny && z < g.nz)
-            d = dout[((long long)b * COUT + co) * g.N + x + (long long)g.nx * (y + (long long)g.ny * z)];
-        dt[i] = d;
-    }
-    __syncthreads();
-    const long long blk = (long long)b * gridDim.x + tile;
-    float* pb = part + blk * (COUT * CIN * 27 + COUT);
-    if (t < CIN * 27) {
-        const int ci = t / 27, tap = t % 27;
-        const int dx = tap % 3, dy = (tap / 3) % 3, dz = tap / 9;
-        float acc[COUT];
 #pragma unroll
-        for (int c = 0; c < COUT; ++c) acc[c] = 0.f;
-        for (int vx = 0; vx < TV; ++vx) {
-            const int lx = vx % TX, ly = (vx / TX) % TY, lz = vx / (TX * TY);
-            const float xv = __bfloat162float(tin[ci * HV + (lx + dx) + HX * ((ly + dy) + HY * (lz + dz))]);
-            if constexpr (COUT % 4 == 0) {
+    for (int k = 0; k < 3; ++k)
+        *reinterpret_cast<uint4*>(tile + k * piece_elems + half_at(v, h)) = *reinterpret_cast<const uint4*>(p[k]);
+}
+
+constexpr int kWgThreads = 288;  // 9 warps, three taps each (dz = w / 3, dy = w % 3)
+
+// Weight and bias gradients: dW[co][ci][tap] = sum_v dout[co][v] in[ci][v + off(tap)], the
+// contraction over voxels as 16 ci x 16 voxels times 16 voxels x 8 co. A block walks the tiles
+// blockIdx.x, + gridDim.x, ... and writes one set of partial sums: part[blk][co][ci * 27 + tap],
+// then part[blk][COUT * CIN * 27 + co].
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(kWgThreads) k_wgrad_mma(const __nv_bfloat16* __restrict__ in,
+                                                          const float* __restrict__ dout, float* __restrict__ part,
+                                                          Grid g, int ntile) {
+    constexpr int NH = COUT > 8 ? 2 : 1;
+    extern __shared__ __align__(16) __nv_bfloat16 wsm[];
+    __nv_bfloat16* at = wsm;                 // [HV][16]
+    __nv_bfloat16* dt = wsm + HV * 16;       // [3][TV][16]
+    const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+    const int tiles = g.tx * g.ty * g.tz;
+    float sum[3][NH][4], bias[8];
 #pragma unroll
-                for (int c = 0; c < COUT; c += 4) {
-                    const float4 d4 = *reinterpret_cast<const float4*>(&dt[vx * COUT + c]);
-                    acc[c] += d4.x * xv;
-                    acc[c + 1] += d4.y * xv;
-                    acc[c + 2] += d4.z * xv;
-                    acc[c + 3] += d4.w * xv;
-                }
-            } else {
+    for (int i = 0; i < 8; ++i) bias[i] = 0.f;
 #pragma unroll
-                for (int c = 0; c < COUT; ++c) acc[c] += dt[vx * COUT + c] * xv;
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int n = 0; n < NH; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sum[k][n][e] = 0.f;
+    for (int it = blockIdx.x; it < ntile; it += gridDim.x) {
+        const int b = it / tiles, tile = it - b * tiles;
+        const int bx = (tile % g.tx) * TX, by = ((tile / g.tx) % g.ty) * TY, bz = (tile / (g.tx * g.ty)) * TZ;
+        const __nv_bfloat16* inb = in + (long long)b * CIN * g.N;
+        const float* db = dout + (long long)b * COUT * g.N;
+        for (int i = t; i < 2 * HV; i += kWgThreads) {
+            const int v = i >> 1, h = i & 1;
+            const int hx = v % HX, hy = (v / HX) % HY, hz = v / (HX * HY);
+            const long long at0 = wrap_any(bx + hx - 1, g.nx) +
+                                  (long long)g.nx * (wrap_any(by + hy - 1, g.ny) + (long long)g.ny * wrap_any(bz + hz - 1, g.nz));
+            __align__(16) __nv_bfloat16 c[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                c[j] = h * 8 + j < CIN ? inb[(long long)(h * 8 + j) * g.N + at0] : __float2bfloat16(0.f);
+            *reinterpret_cast<uint4*>(at + half_at(v, h)) = *reinterpret_cast<const uint4*>(c);
+        }
+        for (int i = t; i < 2 * TV; i += kWgThreads) {  // h = i & 1 = t & 1: one half per thread
+            const int v = i >> 1, h = i & 1;
+            const int x = bx + v % TX, y = by + (v / TX) % TY, z = bz + v / (TX * TY);
+            const bool inside = x < g.nx && y < g.ny && z < g.nz;  // others contribute nothing
+            const long long at0 = x + (long long)g.nx * (y + (long long)g.ny * z);
+            float d[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                d[j] = inside && h * 8 + j < COUT ? db[(long long)(h * 8 + j) * g.N + at0] : 0.f;
+                bias[j] += d[j];
+            }
+            put_pieces(dt, TV * 16, v, h, d);
+        }
+        __syncthreads();
+        float acc[3][NH][4];
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int n = 0; n < NH; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[k][n][e] = 0.f;
+        const int mi = lane >> 3, row = lane & 7;
+        const int dz = w / 3, dy = w % 3;
+        for (int k0 = 0; k0 < TV; k0 += 16) {  // rows of 8 voxels: (ly, lz) and (ly + 1, lz)
+            const int ly = (k0 / TX) % TY, lz = k0 / (TX * TY);
+            uint32_t bf[3][4];
+#pragma unroll
+            for (int p = 0; p < 3; ++p) ldm4t(bf[p], dt + p * TV * 16 + half_at(k0 + (mi & 1) * 8 + row, mi >> 1));
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx) {
+                uint32_t af[4];
+                ldm4t(af, at + half_at(dx + row + HX * (ly + (mi >> 1) + dy + HY * (lz + dz)), mi & 1));
+#pragma unroll
+                for (int p = 0; p < 3; ++p)
+#pragma unroll
+                    for (int n = 0; n < NH; ++n) mma16816(acc[dx][n], af, bf[p][2 * n], bf[p][2 * n + 1]);
             }
         }
 #pragma unroll
-        for (int c = 0; c < COUT; ++c) pb[c * CIN * 27 + t] = acc[c];
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int n = 0; n < NH; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sum[k][n][e] += acc[k][n][e];
+        __syncthreads();
     }
+    float* pb = part + (long long)blockIdx.x * (COUT * CIN * 27 + COUT);
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int n = 0; n < NH; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int ci = (lane >> 2) + 8 * (e >> 1), co = 8 * n + 2 * (lane & 3) + (e & 1);
+                if (ci < CIN && co < COUT) pb[(co * CIN + ci) * 27 + 3 * w + k] = sum[k][n][e];
+            }
+    float(*bsum)[8] = reinterpret_cast<float(*)[8]>(wsm);  // the tiles are read no more
+#pragma unroll
+    for (int j = 0; j < 8; ++j) bsum[t][j] = bias[j];
+    __syncthreads();
     if (t < COUT) {
         float s = 0.f;
-        for (int vx = 0; vx < TV; ++vx) s += dt[vx * COUT + t];
+        for (int i = t >> 3; i < kWgThreads; i += 2) s += bsum[i][t & 7];
         pb[COUT * CIN * 27 + t] = s;
     }
 }
 
-// grad[i] = sum over blocks of part[blk][i], blocks in order
-__global__ void k_reduce_parts(const float* __restrict__ part, int nblk, int n, float* __restrict__ grad) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// Backward data of a 16 -> 16 layer: out[c][v] = (mask > 0) sum_k sum_tap W[k][c][tap] din[k][v - off(tap)],
+// 16 voxels x 16 k times 16 k x 8 c per tap; Wt as k_transpose_w writes it ([c][k][26 - tap], so
+// that the sum reads din[v + off]). One block per tile, two groups of 16 voxels per warp.
+constexpr int kDgSmem = (3 * HV * 16 + 27 * 256) * 2;
+__global__ void __launch_bounds__(256) k_dgrad_mma(const float* __restrict__ din, const __nv_bfloat16* __restrict__ Wt,
+                                                   float* __restrict__ out, const __nv_bfloat16* __restrict__ mask,
+                                                   Grid g) {
+    extern __shared__ __align__(16) __nv_bfloat16 wsm[];
+    __nv_bfloat16* dt = wsm;                      // [3][HV][16]
+    __nv_bfloat16* ws = wsm + 3 * HV * 16;        // [27][lane][n half][k half][2]
+    const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+    const int tile = blockIdx.x, b = blockIdx.y;
+    const int bx = (tile % g.tx) * TX, by = ((tile / g.tx) % g.ty) * TY, bz = (tile / (g.tx * g.ty)) * TZ;
+    const float* db = din + (long long)b * 16 * g.N;
+    for (int i = t; i < 27 * 256; i += 256) {
+        const int tap = i >> 8, l = (i >> 3) & 31, n = (i >> 2) & 1, kh = (i >> 1) & 1, e = i & 1;
+        const int c = 8 * n + (l >> 2), k = 8 * kh + 2 * (l & 3) + e;
+        ws[i] = Wt[(c * 16 + k) * 27 + tap];
+    }
+    for (int i = t; i < 2 * HV; i += 256) {
+        const int v = i >> 1, h = i & 1;
+        const int hx = v % HX, hy = (v / HX) % HY, hz = v / (HX * HY);
+        const long long at0 = wrap_any(bx + hx - 1, g.nx) +
+                              (long long)g.nx * (wrap_any(by + hy - 1, g.ny) + (long long)g.ny * wrap_any(bz + hz - 1, g.nz));
+        float d[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) d[j] = db[(long long)(h * 8 + j) * g.N + at0];
+        put_pieces(dt, HV * 16, v, h, d);
+    }
+    __syncthreads();
+    const int mi = lane >> 3, row = lane & 7;
+    float acc[2][2][4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
+    // group m of the warp: voxel rows ly, ly + 1 of plane lz
+    const int lz = w >> 1, ly0 = (w & 1) * 4;
+#pragma unroll 1
+    for (int tap = 0; tap < 27; ++tap) {
+        const int dx = tap % 3, dy = (tap / 3) % 3, dz = tap / 9;
+        const uint4 bw = *reinterpret_cast<const uint4*>(ws + tap * 256 + lane * 8);
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            const int v = dx + row + HX * (ly0 + 2 * m + (mi & 1) + dy + HY * (lz + dz));
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+                uint32_t af[4];
+                ldm4(af, dt + p * HV * 16 + half_at(v, mi >> 1));
+                mma16816(acc[m][0], af, bw.x, bw.y);
+                mma16816(acc[m][1], af, bw.z, bw.w);
+            }
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int x = bx + (lane >> 2), y = by + ly0 + 2 * m + (e >> 1), z = bz + lz;
+                if (x >= g.nx || y >= g.ny || z >= g.nz) continue;
+                const int c = 8 * n + 2 * (lane & 3) + (e & 1);
+                const long long idx = ((long long)b * 16 + c) * g.N + x + (long long)g.nx * (y + (long long)g.ny * z);
+                out[idx] = __bfloat162float(mask[idx]) <= 0.f ? 0.f : acc[m][n][e];
+            }
+}
+
+// grad[i] = sum over blocks of part[blk][i]: 8 threads per value add contiguous eighths of the
+// blocks in order, then the eighths are added in order.
+__global__ void __launch_bounds__(256) k_reduce_parts(const float* __restrict__ part, int nblk, int n,
+                                                      float* __restrict__ grad) {
+    __shared__ float sm[8][32];
+    const int l = threadIdx.x & 31, seg = threadIdx.x >> 5, i = blockIdx.x * 32 + l;
     float s = 0.f;
-    for (int k = 0; k < nblk; ++k) s += part[(long long)k * n + i];
-    grad[i] = s;
+    if (i < n) {
+        const int k1 = (int)((long long)nblk * (seg + 1) / 8);
+#pragma unroll 4
+        for (int k = (int)((long long)nblk * seg / 8); k < k1; ++k) s += part[(long long)k * n + i];
+    }
+    sm[seg][l] = s;
+    __syncthreads();
+    if (seg == 0 && i < n) {
+        s = sm[0][l];
+#pragma unroll
+        for (int k = 1; k < 8; ++k) s += sm[k][l];
+        grad[i] = s;
+    }
 }
 
 // transposed, flipped weights of one layer: Wt[ci][co][26 - tap] = W[co][ci][tap]
@@ -362,11 +536,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr)
         : "memory");
-}
-
-__device__ __forceinline__ int wrap_any(int i, int n) {
-    i %= n;
-    return i < 0 ? i + n : i;
 }
 
 // out (B x COUT x N) = act(conv(in (B x CIN x N)) + bias); W bf16 [COUT][CIN][27];
@@ -644,7 +813,9 @@ int loss_and_grad(qg_learned L, const Grid& g, int B, const double* R, long long
     k_scale_f<<<148 * 8, 256, 0, st>>>(dp, (long long)B * g.N, acc2 + 2 * nlb);
 
     const dim3 grid(g.tx * g.ty * g.tz, B);
-    const int nblk = grid.x * grid.y;
+    const long long ntile = (long long)grid.x * grid.y;
+    if (ntile > 0x7fffffffLL) return QG_ERR_UNSUPPORTED;
+    const int nblk = (int)std::min<long long>(ntile, 148 * 2);  // blocks of the weight gradients, tiles in turn
     const int maxl = 16 * 16 * 27 + 16;
     QG_TRY(L->part.reserve((size_t)nblk * maxl * sizeof(float)));
     float* part = L->part.as<float>();
@@ -654,21 +825,25 @@ int loss_and_grad(qg_learned L, const Grid& g, int B, const double* R, long long
     for (int l = 0; l < kLayers; ++l)
         k_transpose_w<<<(wcount(l) + 255) / 256, 256, 0, st>>>(W + woff(l), kCin[l], kCout[l],
                                                                 L->wtbf.as<__nv_bfloat16>() + woff(l));
+    constexpr int kWgSmem = (HV + 3 * TV) * 32;
+    static_assert(kWgSmem <= 48 * 1024, "no opt-in");
+    auto reduce = [&](int l) { k_reduce_parts<<<(lsize(l) + 31) / 32, 256, 0, st>>>(part, nblk, lsize(l), G + woff(l)); };
+    if (qg::allow_max_dynamic_smem(k_dgrad_mma) != cudaSuccess) return QG_ERR_CUDA;
     // layer 4 (16 -> 1, linear)
-    k_conv_wgrad<16, 1, __nv_bfloat16><<<grid, 448, 0, st>>>(a[3], dp, part, g);
-    k_reduce_parts<<<(lsize(3) + 255) / 256, 256, 0, st>>>(part, nblk, lsize(3), G + woff(3));
+    k_wgrad_mma<16, 1><<<nblk, kWgThreads, kWgSmem, st>>>(a[3], dp, part, g, (int)ntile);
+    reduce(3);
     k_conv_fwd<1, 16, false, float, float><<<grid, TV, 0, st>>>(dp, Wt + woff(3), nullptr, dA, a[3], g);
     // layer 3 (16 -> 16)
-    k_conv_wgrad<16, 16, __nv_bfloat16><<<grid, 448, 0, st>>>(a[2], dA, part, g);
-    k_reduce_parts<<<(lsize(2) + 255) / 256, 256, 0, st>>>(part, nblk, lsize(2), G + woff(2));
-    k_conv_fwd<16, 16, false, float, float><<<grid, TV, 0, st>>>(dA, Wt + woff(2), nullptr, dB, a[2], g);
+    k_wgrad_mma<16, 16><<<nblk, kWgThreads, kWgSmem, st>>>(a[2], dA, part, g, (int)ntile);
+    reduce(2);
+    k_dgrad_mma<<<grid, 256, kDgSmem, st>>>(dA, Wt + woff(2), dB, a[2], g);
     // layer 2 (16 -> 16)
-    k_conv_wgrad<16, 16, __nv_bfloat16><<<grid, 448, 0, st>>>(a[1], dB, part, g);
-    k_reduce_parts<<<(lsize(1) + 255) / 256, 256, 0, st>>>(part, nblk, lsize(1), G + woff(1));
-    k_conv_fwd<16, 16, false, float, float><<<grid, TV, 0, st>>>(dB, Wt + woff(1), nullptr, dA, a[1], g);
+    k_wgrad_mma<16, 16><<<nblk, kWgThreads, kWgSmem, st>>>(a[1], dB, part, g, (int)ntile);
+    reduce(1);
+    k_dgrad_mma<<<grid, 256, kDgSmem, st>>>(dB, Wt + woff(1), dA, a[1], g);
     // layer 1 (2 -> 16)
-    k_conv_wgrad<2, 16, __nv_bfloat16><<<grid, 448, 0, st>>>(a[0], dA, part, g);
-    k_reduce_parts<<<(lsize(0) + 255) / 256, 256, 0, st>>>(part, nblk, lsize(0), G + woff(0));
+    k_wgrad_mma<2, 16><<<nblk, kWgThreads, kWgSmem, st>>>(a[0], dA, part, g, (int)ntile);
+    reduce(0);
     QG_CUDA_TRY(cudaGetLastError());
     return QG_OK;
 }
