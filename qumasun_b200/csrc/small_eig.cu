@@ -31,6 +31,7 @@ namespace qg {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kHegThreads = 512;  // k_small_heg: a thread per 2 x 2 block of pairs (406 at 56 rows)
 constexpr int kMaxSweeps = 40;
 
 struct SmemEig {
@@ -324,26 +325,25 @@ __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -
 
 struct SmemHeg {
     double2* C;   // k*k working matrix (row-major, Hermitian)
-    double2* C2;  // k*k second buffer of the Jacobi rounds
     double2* L;   // k*k Cholesky factor (lower)
     double2* Q;   // k*k eigenvectors (columns)
-    double2* jd;  // k    U(i, i) of the current round
-    double2* jo;  // k    U(partner(i), i)
+    double2* ph;  // 2 k/2  e^{-i phi} of the pairs of two rounds
+    double2* cs;  // 2 k/2  {cos, sin}
     double* d;    // k    equilibration
-    int* part;    // k
+    int2* pq;     // 2 k/2  the pairs (q = k: none)
     int* rank;    // k
 };
 
 __device__ void layout_heg(SmemHeg& m, double2* base, int k) {
     m.C = base;
-    m.C2 = m.C + k * k;
-    m.L = m.C2 + k * k;
+    m.L = m.C + k * k;
     m.Q = m.L + k * k;
-    m.jd = m.Q + k * k;
-    m.jo = m.jd + k;
-    m.d = reinterpret_cast<double*>(m.jo + k);
-    m.part = reinterpret_cast<int*>(m.d + k);
-    m.rank = m.part + k;
+    m.ph = m.Q + k * k;
+    const int k2 = (k + 1) / 2 * 2;
+    m.cs = m.ph + k2;
+    m.d = reinterpret_cast<double*>(m.cs + k2);
+    m.pq = reinterpret_cast<int2*>(m.d + k2);
+    m.rank = reinterpret_cast<int*>(m.pq + k2);
 }
 
 // Loads the lower triangles of A and B (column-major, lda), equilibrates with
@@ -399,14 +399,17 @@ __device__ bool heg_factor_and_reduce(const double2* __restrict__ A, const doubl
     }
     // Y = L^-1 C, then Y^H; twice: (L^-1 (L^-1 C)^H)^H = L^-1 C L^-H
     for (int pass = 0; pass < 2; ++pass) {
-        for (int col = t; col < k; col += nt) {
-            for (int i = 0; i < k; ++i) {
-                double2 v = m.C[i * k + col];
-                for (int l = 0; l < i; ++l) v = csub(v, cmul(m.L[i * k + l], m.C[l * k + col]));
-                m.C[i * k + col] = cscale(v, 1.0 / m.L[i * k + i].x);
+        // row by row over all columns at once: a thread per column walked 48 dependent sums
+        for (int i = 0; i < k; ++i) {
+            const double inv = 1.0 / m.L[i * k + i].x;
+            for (int col = t; col < k; col += nt) m.C[i * k + col] = cscale(m.C[i * k + col], inv);
+            __syncthreads();
+            for (int e = t; e < (k - i - 1) * k; e += nt) {
+                const int l = i + 1 + e / k, col = e % k;
+                m.C[l * k + col] = csub(m.C[l * k + col], cmul(m.L[l * k + i], m.C[i * k + col]));
             }
+            __syncthreads();
         }
-        __syncthreads();
         for (int e = t; e < k * k; e += nt) {  // conjugate transpose in place
             const int i = e / k, j = e % k;
             if (i < j) {
@@ -435,18 +438,31 @@ __device__ bool heg_factor_and_reduce(const double2* __restrict__ A, const doubl
 }
 
 // Cyclic parallel Jacobi on the Hermitian matrix m.C: round-robin pairs, all
-// rotations of a round applied at once as C' = U^H C U (each new element from four
-// old ones); Q <- Q U. Returns false at the sweep limit.
+// rotations of a round applied at once as C' = U^H C U, Q <- Q U, with U = diag(1, e^{-i phi})
+// [[c, s], [-s, c]] on a pair (p, q). A thread takes the 2 x 2 block of two pairs, in place (the upper
+// blocks; the lower ones are their conjugates). Bound: the latency of a round (two square roots and
+// divisions in a row, then a block), so warp 0 forms the rotations of a round while the other warps
+// turn Q by those of the round before. Eight pencils of 48 columns: 0.78 ms (one matrix element
+// per thread and round, C in two buffers: 2.54 ms). Returns false at the sweep limit.
 __device__ bool heg_jacobi(int k, SmemHeg& m) {
     const int t = threadIdx.x, nt = blockDim.x;
     const int lane = t & 31, warp = t >> 5, nw = nt >> 5;
     const int kk = (k + 1) & ~1;
     const int mm = kk - 1;
     const int npairs = kk / 2;
-    __shared__ double red_off[kThreads / 32], red_tot[kThreads / 32];
+    __shared__ double red_off[kHegThreads / 32], red_tot[kHegThreads / 32];
     __shared__ int done;
     double2* C = m.C;
-    double2* C2 = m.C2;
+    // block (P, R), P <= R, of pairs P and R: e = R (R + 1) / 2 + P
+    const int nblk = npairs * (npairs + 1) / 2;
+    auto block_row = [](int e) {
+        int R = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
+        while ((R + 1) * (R + 2) / 2 <= e) ++R;
+        while (R * (R + 1) / 2 > e) --R;
+        return R;
+    };
+    auto block_col = [&](int e) { const int R = block_row(e); return e - R * (R + 1) / 2; };
+    const int R0 = block_row(t), P0 = block_col(t);
     for (int sweep = 0; sweep < kMaxSweeps; ++sweep) {
         double so = 0.0, st = 0.0;
         for (int i = warp; i < k; i += nw)
@@ -474,87 +490,110 @@ __device__ bool heg_jacobi(int k, SmemHeg& m) {
             done = (off <= 1e-26 * tot || off == 0.0) ? 1 : 0;
         }
         __syncthreads();
-        if (done) {
-            m.C = C;
-            m.C2 = C2;
-            return true;
-        }
+        if (done) return true;
+        // Q <- Q U by the rotations in buffer b, rows w0, w0 + dw, ...; a lane is a pair
+        auto turn_q = [&](int b, int w0, int dw) {
+            if (lane >= npairs) return;
+            const int2 pq = m.pq[b * npairs + lane];
+            if (pq.y >= k) return;
+            const double2 c = m.cs[b * npairs + lane], h = m.ph[b * npairs + lane];
+            for (int row = w0; row < k; row += dw) {
+                const double2 x = m.Q[row * k + pq.x], y = cmul(m.Q[row * k + pq.y], h);
+                m.Q[row * k + pq.x] = csub(cscale(x, c.x), cscale(y, c.y));
+                m.Q[row * k + pq.y] = cadd(cscale(x, c.y), cscale(y, c.x));
+            }
+        };
         for (int round = 0; round < mm; ++round) {
-            for (int pi = t; pi < npairs; pi += nt) {
-                const int a = (pi == 0) ? 0 : ((pi - 1 + round) % mm) + 1;
-                const int b = ((kk - 2 - pi + round) % mm) + 1;
-                const int p = a < b ? a : b, q = a < b ? b : a;
-                if (q < k) {
-                    double c = 1.0, sn = 0.0;
-                    double2 ph = make_double2(1.0, 0.0);  // e^{-i phi}
-                    const double2 cpq = C[p * k + q];
-                    const double apq = hypot(cpq.x, cpq.y);
-                    if (apq != 0.0) {
-                        ph = make_double2(cpq.x / apq, -cpq.y / apq);
-                        const double th = (C[q * k + q].x - C[p * k + p].x) / (2.0 * apq);
-                        const double tt = (th >= 0.0 ? 1.0 : -1.0) / (fabs(th) + sqrt(1.0 + th * th));
-                        c = 1.0 / sqrt(1.0 + tt * tt);
-                        sn = tt * c;
+            const int buf = round & 1;
+            const int2* bpq = m.pq + buf * npairs;
+            const double2 *bph = m.ph + buf * npairs, *bcs = m.cs + buf * npairs;
+            if (warp == 0) {
+                if (lane < npairs) {
+                    const int a = (lane == 0) ? 0 : ((lane - 1 + round) % mm) + 1;
+                    const int b = ((kk - 2 - lane + round) % mm) + 1;
+                    const int p = a < b ? a : b, q = a < b ? b : a;
+                    double2 cs = make_double2(1.0, 0.0), ph = make_double2(1.0, 0.0);
+                    if (q < k) {
+                        const double2 cpq = C[p * k + q];
+                        const double a2 = cpq.x * cpq.x + cpq.y * cpq.y;
+                        if (a2 != 0.0) {
+                            // t = sgn(d) h / (|d| + sqrt(d^2 + h^2)), d = C_qq - C_pp, h = 2 |C_pq|
+                            const double d = C[q * k + q].x - C[p * k + p].x;
+                            const double root = sqrt(d * d + 4.0 * a2), apq = sqrt(a2);
+                            const double tt = (d >= 0.0 ? 2.0 : -2.0) * apq / (fabs(d) + root);
+                            const double inv = 1.0 / apq;
+                            ph = make_double2(cpq.x * inv, -cpq.y * inv);
+                            cs.x = 1.0 / sqrt(1.0 + tt * tt);
+                            cs.y = tt * cs.x;
+                        }
                     }
-                    // U = diag(1, e^{-i phi}) J, J = [[c, s], [-s, c]] on (p, q)
-                    m.part[p] = q;
-                    m.part[q] = p;
-                    m.jd[p] = make_double2(c, 0.0);    // U(p, p)
-                    m.jo[p] = cscale(ph, -sn);         // U(q, p)
-                    m.jd[q] = cscale(ph, c);           // U(q, q)
-                    m.jo[q] = make_double2(sn, 0.0);   // U(p, q)
-                } else if (p < k) {
-                    m.part[p] = -1;
-                    m.jd[p] = make_double2(1.0, 0.0);
-                    m.jo[p] = make_double2(0.0, 0.0);
+                    m.pq[buf * npairs + lane] = make_int2(p, q);
+                    m.ph[buf * npairs + lane] = ph;
+                    m.cs[buf * npairs + lane] = cs;
+                }
+            } else if (round > 0) {
+                turn_q(buf ^ 1, warp - 1, nw - 1);
+            }
+            __syncthreads();
+            for (int e = t; e < nblk; e += nt) {
+                const int P = e == t ? P0 : block_col(e), R = e == t ? R0 : block_row(e);
+                const int2 rp = bpq[P], rq = bpq[R];
+                const double2 hp = bph[P], hq = bph[R], cp = bcs[P], cq = bcs[R];
+                const bool two_r = rp.y < k, two_c = rq.y < k;
+                const double2 zero = make_double2(0.0, 0.0);
+                double2 x[2][2];
+                x[0][0] = C[rp.x * k + rq.x];
+                x[0][1] = two_c ? C[rp.x * k + rq.y] : zero;
+                x[1][0] = two_r ? C[rp.y * k + rq.x] : zero;
+                x[1][1] = two_r && two_c ? C[rp.y * k + rq.y] : zero;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {  // columns
+                    const double2 a = x[i][0], b = cmul(x[i][1], hq);
+                    x[i][0] = csub(cscale(a, cq.x), cscale(b, cq.y));
+                    x[i][1] = cadd(cscale(a, cq.y), cscale(b, cq.x));
+                }
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {  // rows, with U^H
+                    const double2 a = x[0][j], b = cmulc(hp, x[1][j]);
+                    x[0][j] = csub(cscale(a, cp.x), cscale(b, cp.y));
+                    x[1][j] = cadd(cscale(a, cp.y), cscale(b, cp.x));
+                }
+                if (P == R) {  // the pair's own block: real diagonal, Hermitian
+                    x[0][0].y = 0.0;
+                    x[1][1].y = 0.0;
+                    x[1][0] = cconj(x[0][1]);
+                }
+                C[rp.x * k + rq.x] = x[0][0];
+                if (two_c) C[rp.x * k + rq.y] = x[0][1];
+                if (two_r) C[rp.y * k + rq.x] = x[1][0];
+                if (two_r && two_c) C[rp.y * k + rq.y] = x[1][1];
+                if (P != R) {
+                    C[rq.x * k + rp.x] = cconj(x[0][0]);
+                    if (two_c) C[rq.y * k + rp.x] = cconj(x[0][1]);
+                    if (two_r) C[rq.x * k + rp.y] = cconj(x[1][0]);
+                    if (two_r && two_c) C[rq.y * k + rp.y] = cconj(x[1][1]);
                 }
             }
             __syncthreads();
-            // C2(i, j) = sum_{a in {i, ip}, b in {j, jp}} conj(U(a, i)) C(a, b) U(b, j)
-            for (int i = warp; i < k; i += nw) {
-                const int ip = m.part[i];
-                const double2 di = m.jd[i], oi = m.jo[i];
-                for (int j = lane; j < k; j += 32) {
-                    const int jp = m.part[j];
-                    const double2 dj = m.jd[j], oj = m.jo[j];
-                    double2 v = cmulc(di, cmul(C[i * k + j], dj));
-                    if (ip >= 0) v = cadd(v, cmulc(oi, cmul(C[ip * k + j], dj)));
-                    if (jp >= 0) v = cadd(v, cmulc(di, cmul(C[i * k + jp], oj)));
-                    if (ip >= 0 && jp >= 0) v = cadd(v, cmulc(oi, cmul(C[ip * k + jp], oj)));
-                    C2[i * k + j] = v;
-                }
-            }
-            // Q(r, j) <- Q(r, j) U(j, j) + Q(r, jp) U(jp, j), both columns of a pair together
-            for (int i = warp; i < k; i += nw) {
-                for (int j = lane; j < k; j += 32) {
-                    const int jp = m.part[j];
-                    if (jp > j) {
-                        const double2 qj = m.Q[i * k + j], qp = m.Q[i * k + jp];
-                        m.Q[i * k + j] = cadd(cmul(qj, m.jd[j]), cmul(qp, m.jo[j]));
-                        m.Q[i * k + jp] = cadd(cmul(qj, m.jo[jp]), cmul(qp, m.jd[jp]));
-                    }
-                }
-            }
-            __syncthreads();
-            double2* tmp = C;
-            C = C2;
-            C2 = tmp;
         }
+        turn_q((mm - 1) & 1, warp, nw);
+        __syncthreads();
     }
-    m.C = C;
-    m.C2 = C2;
     return false;
 }
 
 // z = D L^-H q for every column, sorted by eigenvalue.
 __device__ void heg_back_transform(int k, SmemHeg& m, double2* __restrict__ Z, int ldz, double* __restrict__ w) {
     const int t = threadIdx.x, nt = blockDim.x;
-    for (int col = t; col < k; col += nt) {  // L^H y = q, backward
-        for (int i = k - 1; i >= 0; --i) {
-            double2 v = m.Q[i * k + col];
-            for (int l = i + 1; l < k; ++l) v = csub(v, cmulc(m.L[l * k + i], m.Q[l * k + col]));
-            m.Q[i * k + col] = cscale(v, 1.0 / m.L[i * k + i].x);
+    for (int i = k - 1; i >= 0; --i) {  // L^H y = q, backward, all columns at once
+        const double inv = 1.0 / m.L[i * k + i].x;
+        for (int col = t; col < k; col += nt) m.Q[i * k + col] = cscale(m.Q[i * k + col], inv);
+        __syncthreads();
+        for (int e = t; e < i * k; e += nt) {
+            const int l = e / k, col = e % k;
+            m.Q[l * k + col] = csub(m.Q[l * k + col], cmulc(m.L[i * k + l], m.Q[i * k + col]));
         }
+        __syncthreads();
     }
     for (int i = t; i < k; i += nt) {
         const double li = m.C[i * k + i].x;
@@ -573,7 +612,7 @@ __device__ void heg_back_transform(int k, SmemHeg& m, double2* __restrict__ Z, i
     for (int i = t; i < k; i += nt) w[m.rank[i]] = m.C[i * k + i].x;
 }
 
-__global__ void __launch_bounds__(kThreads) k_small_heg(const double2* __restrict__ A, const double2* __restrict__ B,
+__global__ void __launch_bounds__(kHegThreads) k_small_heg(const double2* __restrict__ A, const double2* __restrict__ B,
                                                          int lda, long long stride_ab, int k,
                                                          const int* __restrict__ skip, double2* Z, int ldz,
                                                          long long stride_z, double* __restrict__ w,
@@ -603,7 +642,9 @@ __global__ void __launch_bounds__(kThreads) k_small_heg(const double2* __restric
 }  // namespace
 
 size_t small_heg_smem(int k) {
-    return (size_t)(4 * k * k + 2 * k) * sizeof(double2) + (size_t)k * sizeof(double) + (size_t)2 * k * sizeof(int);
+    const int k2 = (k + 1) / 2 * 2;
+    return (size_t)(3 * k * k + 2 * k2) * sizeof(double2) + (size_t)k2 * (sizeof(double) + sizeof(int2)) +
+           (size_t)k * sizeof(int);
 }
 
 int small_heg_launch(const double2* A, const double2* B, int lda, long long stride_ab, int k, const int* skip,
@@ -613,7 +654,7 @@ int small_heg_launch(const double2* A, const double2* B, int lda, long long stri
     const size_t smem = small_heg_smem(k);
     if (smem > 48 * 1024)
         QG_CUDA_TRY(allow_max_dynamic_smem(k_small_heg));
-    k_small_heg<<<batch, kThreads, smem, st>>>(A, B, lda, stride_ab, k, skip, Z, ldz, stride_z, w, stride_w, info,
+    k_small_heg<<<batch, kHegThreads, smem, st>>>(A, B, lda, stride_ab, k, skip, Z, ldz, stride_z, w, stride_w, info,
                                                pivot_floor);
     QG_CUDA_TRY(cudaGetLastError());
     return QG_OK;

@@ -14,7 +14,7 @@ int small_eig_launch(const double* A, const double* B, int lda, long long stride
                      int ldz, long long stride_z, double* w, long long stride_w, int* info, int batch,
                      cudaStream_t st);
 
-constexpr int kSmallHegMax = 56;  // largest complex pencil (4 k x k complex matrices in shared memory)
+constexpr int kSmallHegMax = 56;  // largest complex pencil (3 k x k complex matrices in shared memory)
 
 // Complex Hermitian counterpart (replaces lapack_ZHEGVX, w_zhegvx.h:24-107, for the
 // k-point LOBPCG pencils): batch problems A_b z = lambda B_b z, k x k complex
