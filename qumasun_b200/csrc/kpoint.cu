@@ -7,8 +7,8 @@
 // Launches for a block of states, as on the real path: the projection and the scatter on the
 // tensor cores (nonlocal.cu: Bloch phases of the grid points and of the periodic images, the
 // projector tables of the real path), and between them
-//   k_stencil_tma   V u - 1/2 (Lap + 2i g.grad - g^2) u, both parts of a plane staged together
-//                   (stencil_tma.cu, NC = 2); any other shape runs k_kpoint_plain
+//   k_stencil_kpoint  V u - 1/2 (Lap + 2i g.grad - g^2) u, both parts of a plane staged together
+//                   (stencil_kpoint.cu); any other shape runs k_kpoint_plain
 #include <algorithm>
 #include <cmath>
 
@@ -193,7 +193,7 @@ int apply_hamiltonian_zk(qg_hamiltonian h, int nk, const double* kv, int nsk, co
     }
     if (pt) pt->mark(1, st);
     constexpr int PX = 16 / sizeof(T);
-    if (h->stencil_variant == 1 || !stencil_tma_ok<T>(a, h->order, 2) || (nk > 1 && (ldk % PX || ldkh % PX))) {
+    if (h->stencil_variant == 1 || !stencil_kpoint_ok<T>(a, h->order) || (nk > 1 && (ldk % PX || ldkh % PX))) {
         dim3 g((unsigned)((N + 255) / 256), (unsigned)(nk * nsk));
         switch (h->order) {
             case 2: k_kpoint_plain<T, 2><<<g, 256, 0, st>>>(a); break;
@@ -201,7 +201,7 @@ int apply_hamiltonian_zk(qg_hamiltonian h, int nk, const double* kv, int nsk, co
             default: k_kpoint_plain<T, 8><<<g, 256, 0, st>>>(a); break;
         }
     } else {
-        QG_TRY(launch_stencil_tma<T>(a, h->order, st, 2));
+        QG_TRY(launch_stencil_kpoint<T>(a, h->order, st));
     }
     if (pt) pt->mark(2, st);
     if (nonlocal) QG_TRY(brick_scatter_z<T>(h, nk, nsk, HX, ldhx, ldkh, phase, scratch, st));

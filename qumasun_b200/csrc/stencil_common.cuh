@@ -26,7 +26,7 @@ struct HamArgs {
     // axis whose |g| < 1e-8), c0 then carries the -coef*|g|^2 term
     long long xim, hxim;
     T dx[4], dy[4], dz[4];
-    // several k-points in one launch (NC = 2): states are grouped by k, nsk per k;
+    // several k-points in one launch: states are grouped by k, nsk per k;
     // state s of k-point k starts at X + k*ldkx + s*ldx (HX + k*ldkhx + s*ldhx), and
     // kco[k*13 + {0, 1..4, 5..8, 9..12}] replaces c0, dx, dy, dz (nsk = 0: one k-point)
     int nsk;
@@ -48,12 +48,12 @@ __device__ __forceinline__ int wrap_idx(int i, int n) {
 }
 
 
-// nc = 1: real states; nc = 2: complex k-point states (order 8 only).
+// Real states, one plane and row per consumer step (stencil_tma.cu).
 template <typename T>
-int launch_stencil_tma(const HamArgs<T>& a, int order, cudaStream_t st, int nc = 1);
+int launch_stencil_tma(const HamArgs<T>& a, int order, cudaStream_t st);
 // True when launch_stencil_tma accepts this shape and alignment.
 template <typename T>
-bool stencil_tma_ok(const HamArgs<T>& a, int order, int nc = 1);
+bool stencil_tma_ok(const HamArgs<T>& a, int order);
 // Real states, two output planes per consumer step (stencil_pair.cu).
 template <typename T>
 int launch_stencil_pair(const HamArgs<T>& a, int order, cudaStream_t st);
@@ -65,6 +65,12 @@ template <typename T>
 int launch_stencil_rows(const HamArgs<T>& a, int order, cudaStream_t st, bool vring = true);
 template <typename T>
 bool stencil_rows_ok(const HamArgs<T>& a, int order, bool vring = true);
+
+// Complex k-point states of orders 2, 6 and 8 (stencil_kpoint.cu).
+template <typename T>
+int launch_stencil_kpoint(const HamArgs<T>& a, int order, cudaStream_t st);
+template <typename T>
+bool stencil_kpoint_ok(const HamArgs<T>& a, int order);
 
 // 8th-order periodic FD gradient of the listed real states (sidx, DEVICE) of the nin at X (gradient.cu):
 // component d of state s at out + (d * ns + s) * N (Gradient8th, GridGradient8th.h:19-235).

@@ -121,49 +121,9 @@ __device__ __forceinline__ T lap_point(T c, const T* xm, const T* xp, const T* y
     }
 }
 
-// g.grad of one point with the first derivative of the FD order: 8th (672, -168, 32, -3)/840h,
-// 6th (45, -9, 1)/60h, 2nd 1/2h, grouped as in LaplasianKpoint{8th,6th,2nd}_halo_f
-// (GridDifferenceKpoint8th.h:18-122, 6th.h:19-107, 2nd.h:19-92); the factor 2*coef and g
-// are folded into a.dx/dy/dz.
-template <typename T, int ORDER>
-__device__ __forceinline__ T der_point(const T* xm, const T* xp, const T* ym, const T* yp, const T* zm,
-                                       const T* zp, const HamArgs<T>& a) {
-    if constexpr (ORDER == 2) {
-        T g = a.dx[0] * (xp[0] - xm[0]);
-        g += a.dy[0] * (yp[0] - ym[0]);
-        g += a.dz[0] * (zp[0] - zm[0]);
-        return g;
-    } else if constexpr (ORDER == 6) {
-        T g = a.dx[2] * (xp[2] - xm[2]) + a.dx[1] * (xp[1] - xm[1]) + a.dx[0] * (xp[0] - xm[0]);
-        g += a.dy[2] * (yp[2] - ym[2]) + a.dy[1] * (yp[1] - ym[1]) + a.dy[0] * (yp[0] - ym[0]);
-        g += a.dz[2] * (zp[2] - zm[2]) + a.dz[1] * (zp[1] - zm[1]) + a.dz[0] * (zp[0] - zm[0]);
-        return g;
-    } else {
-        T g = a.dx[3] * (xp[3] - xm[3]) + a.dx[2] * (xp[2] - xm[2]) + a.dx[1] * (xp[1] - xm[1]) + a.dx[0] * (xp[0] - xm[0]);
-        g += a.dy[3] * (yp[3] - ym[3]) + a.dy[2] * (yp[2] - ym[2]) + a.dy[1] * (yp[1] - ym[1]) + a.dy[0] * (yp[0] - ym[0]);
-        g += a.dz[3] * (zp[3] - zm[3]) + a.dz[2] * (zp[2] - zm[2]) + a.dz[1] * (zp[1] - zm[1]) + a.dz[0] * (zp[0] - zm[0]);
-        return g;
-    }
-}
-
-// -1/2 (Lap - g^2) of one point for complex k-point states: orders 6 and 8 as lap_point
-// (a.c0 carrying -coef g^2); order 2 grouped as LaplasianKpoint2nd_halo_f
-// (GridDifferenceKpoint2nd.h:69-72), c0 p + cx (p+x + p-x) + cy (..) + cz (..).
-template <typename T, int ORDER>
-__device__ __forceinline__ T lap_point_k(T c, const T* xm, const T* xp, const T* ym, const T* yp, const T* zm,
-                                         const T* zp, const HamArgs<T>& a) {
-    if constexpr (ORDER == 2) {
-        return a.c0 * c + a.cx[0] * (xp[0] + xm[0]) + a.cy[0] * (yp[0] + ym[0]) + a.cz[0] * (zp[0] + zm[0]);
-    } else {
-        return lap_point<T, ORDER>(c, xm, xp, ym, yp, zm, zp, a);
-    }
-}
-
 constexpr int kBarBytes = 1024;  // mbarriers + control words at the front of dynamic shared memory
 constexpr int kMaxThreads = 448;
 constexpr int kMaxConsumers = 416;
-constexpr int kMaxThreadsKp = 352;  // complex states keep two register windows per thread
-constexpr int kMaxConsumersKp = 320;
 constexpr int kMaxStages = 16;
 
 template <int ORDER>
@@ -179,15 +139,12 @@ struct WorkGrid {
 // Persistent kernel: block b processes work items b, b + gridDim.x, ... where
 // item = (state, y tile, z slab). The plane ring and its phases run on across
 // items, so the producer streams the next item's planes while the consumers
-// finish the current one. NC = 2 carries complex k-point states: a stage holds
-// the real and the imaginary rows of one plane, and each point adds the
-// first-derivative coupling -(1/2) 2i g.grad between the two parts
-// (LaplasianKpoint8th_halo_f, GridDifferenceKpoint8th.h:18-122).
+// finish the current one.
 // NXC > 0: the row length nx as a compile-time constant (instantiated for the common
 // grids), so that the y-neighbour offsets +-d*nx become immediate offsets of the
 // shared-memory loads instead of per-load address arithmetic.
-template <typename T, int ORDER, int PX, int NC, int NXC>
-__global__ void __launch_bounds__(NC == 1 ? kMaxThreads : kMaxThreadsKp, 1)
+template <typename T, int ORDER, int PX, int NXC>
+__global__ void __launch_bounds__(kMaxThreads, 1)
     k_stencil_tma(const HamArgs<T> a, const WorkGrid wg, int nst) {
     constexpr int R = radius<ORDER>();
     constexpr int Q = 2 * R + 1;
@@ -201,8 +158,7 @@ __global__ void __launch_bounds__(NC == 1 ? kMaxThreads : kMaxThreadsKp, 1)
 
     const int nx = NXC > 0 ? NXC : a.nx, ny = a.ny, nz = a.nz, ty = a.ty;
     const int rows = ty + 2 * R;
-    const int comp_elems = rows * nx;  // one part (real or imaginary) of a plane
-    const int stage_elems = NC * comp_elems;
+    const int stage_elems = rows * nx;
     const uint32_t stage_bytes = (uint32_t)stage_elems * sizeof(T);
     const int tpr = nx / PX;
     const int ncons = tpr * ty;
@@ -245,17 +201,13 @@ __global__ void __launch_bounds__(NC == 1 ? kMaxThreads : kMaxThreadsKp, 1)
                     const long long zoff = (long long)wrap_idx(p, nz) * plane;
                     T* dst = ring + (size_t)j * stage_elems;
                     mbar_expect_tx(&full[j], stage_bytes);
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        const T* src = Xs + (c ? a.xim : 0) + zoff;
-                        int r = 0;
-                        while (r < rows) {
-                            const int y = wrap_idx(y0 - R + r, ny);
-                            const int cnt = min(rows - r, ny - y);
-                            bulk_g2s(dst + (size_t)c * comp_elems + (size_t)r * nx, src + (long long)y * nx,
-                                     (uint32_t)(cnt * nx * sizeof(T)), &full[j]);
-                            r += cnt;
-                        }
+                    const T* src = Xs + zoff;
+                    int r = 0;
+                    while (r < rows) {
+                        const int y = wrap_idx(y0 - R + r, ny);
+                        const int cnt = min(rows - r, ny - y);
+                        bulk_g2s(dst + (size_t)r * nx, src + (long long)y * nx, (uint32_t)(cnt * nx * sizeof(T)), &full[j]);
+                        r += cnt;
                     }
                     ctl[1] = pos;
                 }
@@ -293,13 +245,13 @@ __global__ void __launch_bounds__(NC == 1 ? kMaxThreads : kMaxThreadsKp, 1)
             // Register windows addressed by (step mod Q): the z-march is unrolled Q
             // times, so plane z - R + d sits in slot (k + d) % Q at unrolled step k and
             // the windows rotate by renaming instead of register moves (measured 3-13 %
-            // faster for orders 4-8 and complex states; the 3-point order-2 window
+            // faster for orders 4-8; the 3-point order-2 window
             // keeps one step per iteration and shifts, which measured faster there).
             // q holds planes z-R .. z+R of the state, vq the potential of planes z .. z+R.
-            constexpr bool kRot = !(ORDER == 2 && NC == 1);
+            constexpr bool kRot = ORDER != 2;
             constexpr int KU = kRot ? Q : 1;
             auto sl = [](int k, int d) { return kRot ? (k + d) % Q : d; };
-            Vec<T, PX> q[NC][Q];
+            Vec<T, PX> q[Q];
             Vec<T, PX> vq[Q];
             // prologue: own z-window from the item's first 2R planes
             int j = pos % nst;
@@ -308,9 +260,7 @@ __global__ void __launch_bounds__(NC == 1 ? kMaxThreads : kMaxThreadsKp, 1)
 #pragma unroll
             for (int d = 0; d < 2 * R; ++d) {
                 if (w && !mbar_wait(&full[j], ph)) w = false;
-#pragma unroll
-                for (int cc = 0; cc < NC; ++cc)
-                    q[cc][d].v = *reinterpret_cast<const VT*>(ring + j * stage_elems + cc * comp_elems + rowoff + ix0);
+                q[d].v = *reinterpret_cast<const VT*>(ring + j * stage_elems + rowoff + ix0);
                 if (++j == nst) { j = 0; ph ^= 1u; }
             }
             const T* vp = a.V + (long long)zs * plane + col;  // no wrap: zslab >= 2R keeps zs + R - 1 < ze <= nz
@@ -332,18 +282,6 @@ __global__ void __launch_bounds__(NC == 1 ? kMaxThreads : kMaxThreadsKp, 1)
             int jp = j;             // stage of plane z + R (= position pos + 2R)
             uint32_t php = ph;
             T* hxp = a.HX + state_offset(a, s, true) + (long long)zs * plane + col;
-            // per-k-point coefficients of the k-point kinetic term
-            HamArgs<T> ak = a;
-            if (NC == 2 && a.kco) {
-                const T* kc = a.kco + (long long)(s / a.nsk) * 13;
-                ak.c0 = kc[0];
-#pragma unroll
-                for (int d = 0; d < 4; ++d) {
-                    ak.dx[d] = kc[1 + d];
-                    ak.dy[d] = kc[5 + d];
-                    ak.dz[d] = kc[9 + d];
-                }
-            }
             for (int z = zs; z < ze && !bad;) {
 #pragma unroll
             for (int k = 0; k < KU; ++k) {
@@ -355,73 +293,51 @@ __global__ void __launch_bounds__(NC == 1 ? kMaxThreads : kMaxThreadsKp, 1)
                     bad = true;
                     break;
                 }
-                T lap[NC][PX], der[NC][PX];
+                T lap[PX];
+                const T* pzs = ring + jz * stage_elems;
+                const T* pps = ring + jp * stage_elems;
+                q[sl(k, 2 * R)].v = *reinterpret_cast<const VT*>(pps + rowoff + ix0);
+                T xv[(2 * NV + 1) * PX];
 #pragma unroll
-                for (int cc = 0; cc < NC; ++cc) {
-                    const T* pzs = ring + jz * stage_elems + cc * comp_elems;
-                    const T* pps = ring + jp * stage_elems + cc * comp_elems;
-                    q[cc][sl(k, 2 * R)].v = *reinterpret_cast<const VT*>(pps + rowoff + ix0);
-                    T xv[(2 * NV + 1) * PX];
+                for (int v = 0; v < 2 * NV; ++v) {
+                    Vec<T, PX> wv;
+                    wv.v = *reinterpret_cast<const VT*>(pzs + xoff[v]);
+                    const int slot = (v < NV) ? v : v + 1;
 #pragma unroll
-                    for (int v = 0; v < 2 * NV; ++v) {
-                        Vec<T, PX> wv;
-                        wv.v = *reinterpret_cast<const VT*>(pzs + xoff[v]);
-                        const int slot = (v < NV) ? v : v + 1;
+                    for (int e = 0; e < PX; ++e) xv[slot * PX + e] = wv.e[e];
+                }
 #pragma unroll
-                        for (int e = 0; e < PX; ++e) xv[slot * PX + e] = wv.e[e];
-                    }
+                for (int e = 0; e < PX; ++e) xv[NV * PX + e] = q[sl(k, R)].e[e];
+                Vec<T, PX> ypv[R], ymv[R];
 #pragma unroll
-                    for (int e = 0; e < PX; ++e) xv[NV * PX + e] = q[cc][sl(k, R)].e[e];
-                    Vec<T, PX> ypv[R], ymv[R];
+                for (int d = 1; d <= R; ++d) {
+                    ypv[d - 1].v = *reinterpret_cast<const VT*>(pzs + rowoff + ix0 + d * nx);
+                    ymv[d - 1].v = *reinterpret_cast<const VT*>(pzs + rowoff + ix0 - d * nx);
+                }
+#pragma unroll
+                for (int e = 0; e < PX; ++e) {
+                    T xm[R], xp[R], ym[R], yp[R], zm[R], zp[R];
 #pragma unroll
                     for (int d = 1; d <= R; ++d) {
-                        ypv[d - 1].v = *reinterpret_cast<const VT*>(pzs + rowoff + ix0 + d * nx);
-                        ymv[d - 1].v = *reinterpret_cast<const VT*>(pzs + rowoff + ix0 - d * nx);
+                        xm[d - 1] = xv[NV * PX + e - d];
+                        xp[d - 1] = xv[NV * PX + e + d];
+                        ym[d - 1] = ymv[d - 1].e[e];
+                        yp[d - 1] = ypv[d - 1].e[e];
+                        zm[d - 1] = q[sl(k, R - d)].e[e];
+                        zp[d - 1] = q[sl(k, R + d)].e[e];
                     }
-#pragma unroll
-                    for (int e = 0; e < PX; ++e) {
-                        T xm[R], xp[R], ym[R], yp[R], zm[R], zp[R];
-#pragma unroll
-                        for (int d = 1; d <= R; ++d) {
-                            xm[d - 1] = xv[NV * PX + e - d];
-                            xp[d - 1] = xv[NV * PX + e + d];
-                            ym[d - 1] = ymv[d - 1].e[e];
-                            yp[d - 1] = ypv[d - 1].e[e];
-                            zm[d - 1] = q[cc][sl(k, R - d)].e[e];
-                            zp[d - 1] = q[cc][sl(k, R + d)].e[e];
-                        }
-                        if constexpr (NC == 2) {
-                            lap[cc][e] = lap_point_k<T, ORDER>(q[cc][sl(k, R)].e[e], xm, xp, ym, yp, zm, zp, ak);
-                            der[cc][e] = der_point<T, ORDER>(xm, xp, ym, yp, zm, zp, ak);
-                        } else {
-                            lap[cc][e] = lap_point<T, ORDER>(q[cc][sl(k, R)].e[e], xm, xp, ym, yp, zm, zp, ak);
-                        }
-                    }
+                    lap[e] = lap_point<T, ORDER>(q[sl(k, R)].e[e], xm, xp, ym, yp, zm, zp, a);
                 }
                 __syncwarp(wmask);
                 if (lane == 0) mbar_arrive(&empty[jz]);  // plane z is no longer read
-                if constexpr (NC == 1) {
-                    Vec<T, PX> out;
+                Vec<T, PX> out;
 #pragma unroll
-                    for (int e = 0; e < PX; ++e) out.e[e] = vq[sl(k, 0)].e[e] * q[0][sl(k, R)].e[e] + lap[0][e];
-                    *reinterpret_cast<VT*>(hxp) = out.v;
-                } else {
-                    // re: V re + L re - D im;  im: V im + L im + D re
-                    Vec<T, PX> ore, oim;
-#pragma unroll
-                    for (int e = 0; e < PX; ++e) {
-                        ore.e[e] = (vq[sl(k, 0)].e[e] * q[0][sl(k, R)].e[e] + lap[0][e]) - der[1][e];
-                        oim.e[e] = (vq[sl(k, 0)].e[e] * q[1][sl(k, R)].e[e] + lap[1][e]) + der[0][e];
-                    }
-                    *reinterpret_cast<VT*>(hxp) = ore.v;
-                    *reinterpret_cast<VT*>(hxp + a.hxim) = oim.v;
-                }
+                for (int e = 0; e < PX; ++e) out.e[e] = vq[sl(k, 0)].e[e] * q[sl(k, R)].e[e] + lap[e];
+                *reinterpret_cast<VT*>(hxp) = out.v;
                 hxp += plane;
                 if constexpr (!kRot) {
 #pragma unroll
-                    for (int cc = 0; cc < NC; ++cc)
-#pragma unroll
-                        for (int d = 0; d < 2 * R; ++d) q[cc][d] = q[cc][d + 1];
+                    for (int d = 0; d < 2 * R; ++d) q[d] = q[d + 1];
 #pragma unroll
                     for (int d = 0; d < R; ++d) vq[d] = vq[d + 1];
                 }
@@ -454,10 +370,10 @@ __global__ void __launch_bounds__(NC == 1 ? kMaxThreads : kMaxThreadsKp, 1)
 
 // Rows per tile: the largest divisor of ny (<= 16) keeping the consumer threads within the kernel's limit.
 template <typename T>
-int tma_tile_rows(const HamArgs<T>& a, int nc, int order) {
+int tma_tile_rows(const HamArgs<T>& a, int order) {
     constexpr int PX = 16 / sizeof(T);
     // order 2 (3-plane window, DRAM-bound) measured fastest with at most 384 consumers
-    const int maxc = nc == 1 ? (order == 2 ? 384 : kMaxConsumers) : kMaxConsumersKp;
+    const int maxc = order == 2 ? 384 : kMaxConsumers;
     int ty = 0;
     for (int t = 1; t <= 16; ++t)
         if (a.ny % t == 0 && (a.nx / PX) * t <= maxc) ty = t;
@@ -493,29 +409,29 @@ int sm_count() {
 
 namespace {
 
-template <typename T, int ORDER, int NC, int NXC = 0>
+template <typename T, int ORDER, int NXC = 0>
 int launch_order(const HamArgs<T>& a, cudaStream_t st) {
     constexpr int PX = 16 / sizeof(T);
     constexpr int R = radius<ORDER>();
     if constexpr (NXC == 0 && ORDER >= 4) {
         // orders 4-8, FP64 and FP32: row lengths of the common grids compiled in
         switch (a.nx) {
-            case 40: return launch_order<T, ORDER, NC, 40>(a, st);
-            case 80: return launch_order<T, ORDER, NC, 80>(a, st);
-            case 120: return launch_order<T, ORDER, NC, 120>(a, st);
+            case 40: return launch_order<T, ORDER, 40>(a, st);
+            case 80: return launch_order<T, ORDER, 80>(a, st);
+            case 120: return launch_order<T, ORDER, 120>(a, st);
             default: break;
         }
     }
-    const size_t stage = (size_t)NC * (a.ty + 2 * R) * a.nx * sizeof(T);
+    const size_t stage = (size_t)(a.ty + 2 * R) * a.nx * sizeof(T);
     const int nst = ring_stages_for(R, stage);
     if (nst < 0) return QG_ERR_UNSUPPORTED;
     const size_t smem = kBarBytes + (size_t)nst * stage;
-    auto kern = k_stencil_tma<T, ORDER, PX, NC, NXC>;
+    auto kern = k_stencil_tma<T, ORDER, PX, NXC>;
     if (allow_max_dynamic_smem(kern) != cudaSuccess)
         return QG_ERR_UNSUPPORTED;
     const int ncons = (a.nx / PX) * a.ty;
     const int threads = 32 + ncons;
-    if (threads > (NC == 1 ? kMaxThreads : kMaxThreadsKp)) return QG_ERR_UNSUPPORTED;
+    if (threads > kMaxThreads) return QG_ERR_UNSUPPORTED;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess || per_sm < 1)
         return QG_ERR_UNSUPPORTED;
@@ -537,46 +453,37 @@ int launch_order(const HamArgs<T>& a, cudaStream_t st) {
 }  // namespace
 
 template <typename T>
-bool stencil_tma_ok(const HamArgs<T>& a, int order, int nc) {
+bool stencil_tma_ok(const HamArgs<T>& a, int order) {
     constexpr int PX = 16 / sizeof(T);
     const int R = order == 2 ? 1 : (order == 8 ? 4 : 3);
-    if (nc != 1 && nc != 2) return false;
-    if (nc == 2 && ((order != 2 && order != 6 && order != 8) || (a.xim % PX) || (a.hxim % PX))) return false;
     if (a.nx % PX != 0 || ((uintptr_t)a.X % 16) || ((uintptr_t)a.HX % 16) || ((uintptr_t)a.V % 16) ||
         (a.ldx % PX) || (a.ldhx % PX) || !a.err || a.ny < 2 * R || a.nx < 2 * R)
         return false;
-    const int ty = tma_tile_rows(a, nc, order);
+    const int ty = tma_tile_rows(a, order);
     if (ty == 0) return false;
-    const size_t stage = (size_t)nc * (ty + 2 * R) * a.nx * sizeof(T);
+    const size_t stage = (size_t)(ty + 2 * R) * a.nx * sizeof(T);
     return ring_stages_for(R, stage) > 0;
 }
 
 // Returns QG_ERR_UNSUPPORTED (launching nothing) when the shape or alignment
 // does not fit this kernel; the caller then uses the register-window kernel.
 template <typename T>
-int launch_stencil_tma(const HamArgs<T>& a, int order, cudaStream_t st, int nc) {
-    if (!stencil_tma_ok<T>(a, order, nc)) return QG_ERR_UNSUPPORTED;
+int launch_stencil_tma(const HamArgs<T>& a, int order, cudaStream_t st) {
+    if (!stencil_tma_ok<T>(a, order)) return QG_ERR_UNSUPPORTED;
     HamArgs<T> b = a;
-    b.ty = tma_tile_rows(a, nc, order);
-    if (nc == 2) {
-        switch (order) {
-            case 2: return launch_order<T, 2, 2>(b, st);
-            case 6: return launch_order<T, 6, 2>(b, st);
-            default: return launch_order<T, 8, 2>(b, st);
-        }
-    }
+    b.ty = tma_tile_rows(a, order);
     switch (order) {
-        case 2: return launch_order<T, 2, 1>(b, st);
-        case 4: return launch_order<T, 4, 1>(b, st);
-        case 6: return launch_order<T, 6, 1>(b, st);
-        case 8: return launch_order<T, 8, 1>(b, st);
+        case 2: return launch_order<T, 2>(b, st);
+        case 4: return launch_order<T, 4>(b, st);
+        case 6: return launch_order<T, 6>(b, st);
+        case 8: return launch_order<T, 8>(b, st);
         default: return QG_ERR_INVALID;
     }
 }
 
-template bool stencil_tma_ok<double>(const HamArgs<double>&, int, int);
-template bool stencil_tma_ok<float>(const HamArgs<float>&, int, int);
-template int launch_stencil_tma<double>(const HamArgs<double>&, int, cudaStream_t, int);
-template int launch_stencil_tma<float>(const HamArgs<float>&, int, cudaStream_t, int);
+template bool stencil_tma_ok<double>(const HamArgs<double>&, int);
+template bool stencil_tma_ok<float>(const HamArgs<float>&, int);
+template int launch_stencil_tma<double>(const HamArgs<double>&, int, cudaStream_t);
+template int launch_stencil_tma<float>(const HamArgs<float>&, int, cudaStream_t);
 
 }  // namespace qg
