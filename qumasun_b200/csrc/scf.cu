@@ -195,26 +195,51 @@ __global__ void __launch_bounds__(kThreads) k_potential_finish(long long N, doub
 
 // ---------------------------------------------------------------- Taylor-4 propagation
 
-// X += a * W for both parts (REAL_STEP), or X.re += a * W.im, X.im += b * W.re; each
-// product rounded before the add, as the reference's separate loops form them.
-template <bool REAL_STEP>
-__global__ void __launch_bounds__(kThreads) k_td_update(int ns, long long N, double* __restrict__ X, long long ldx,
-                                                        const double* __restrict__ W, long long ldw, double a, double b) {
-    const long long total = (long long)ns * N;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-        const long long s = t / N, i = t - s * N;
-        double* xr = X + s * ldx + i;
-        double* xi = xr + N;
-        const double* wr = W + s * ldw + i;
-        const double* wi = wr + N;
-        if constexpr (REAL_STEP) {
-            *xr = __dadd_rn(*xr, __dmul_rn(a, *wr));
-            *xi = __dadd_rn(*xi, __dmul_rn(a, *wi));
-        } else {
-            const double re = *wr, im = *wi;
-            *xr = __dadd_rn(*xr, __dmul_rn(a, im));
-            *xi = __dadd_rn(*xi, __dmul_rn(b, re));
+// Two Taylor terms in one pass, x = (x + i-term of W1) + real term of W2:
+//   X.re = (X.re + a1 W1.im) + a2 W2.re,  X.im = (X.im + b1 W1.re) + a2 W2.im,
+// each product rounded before its add, as the reference's separate loops form them. blockIdx.y is
+// the state; VEC: two points per thread (N, ldx even and X on 16 bytes). Bound: DRAM, 64 bytes per
+// point. 64 states of 80^3: 0.31 ms for two terms (6.8 TB/s) against 0.58 ms for two passes.
+template <bool VEC>
+__global__ void __launch_bounds__(kThreads) k_td_update2(long long N, double* __restrict__ X, long long ldx,
+                                                         const double* __restrict__ W1, const double* __restrict__ W2,
+                                                         long long ldw, double a1, double b1, double a2) {
+    auto step = [](double x, double c, double w, double d, double v) {
+        return __dadd_rn(__dadd_rn(x, __dmul_rn(c, w)), __dmul_rn(d, v));
+    };
+    double* x = X + blockIdx.y * ldx;
+    const double *w1 = W1 + blockIdx.y * ldw, *w2 = W2 + blockIdx.y * ldw;
+    const long long first = (long long)blockIdx.x * kThreads + threadIdx.x, stride = (long long)gridDim.x * kThreads;
+    if constexpr (VEC) {
+        const long long n2 = N / 2;
+        double2 *xr = reinterpret_cast<double2*>(x), *xi = reinterpret_cast<double2*>(x + N);
+        const double2 *ur = reinterpret_cast<const double2*>(w1), *ui = reinterpret_cast<const double2*>(w1 + N);
+        const double2 *vr = reinterpret_cast<const double2*>(w2), *vi = reinterpret_cast<const double2*>(w2 + N);
+        for (long long i = first; i < n2; i += stride) {
+            const double2 r = xr[i], m = xi[i], a = ur[i], b = ui[i], c = vr[i], d = vi[i];
+            xr[i] = make_double2(step(r.x, a1, b.x, a2, c.x), step(r.y, a1, b.y, a2, c.y));
+            xi[i] = make_double2(step(m.x, b1, a.x, a2, d.x), step(m.y, b1, a.y, a2, d.y));
         }
+    } else {
+        for (long long i = first; i < N; i += stride) {
+            const double a = w1[i], b = w1[N + i];
+            x[i] = step(x[i], a1, b, a2, w2[i]);
+            x[N + i] = step(x[N + i], b1, a, a2, w2[N + i]);
+        }
+    }
+}
+
+static void launch_td_update2(int ns, long long N, double* X, long long ldx, const double* W1, const double* W2,
+                              long long ldw, double a1, double b1, double a2, cudaStream_t st) {
+    const bool vec = N % 2 == 0 && ldx % 2 == 0 && (uintptr_t)X % 16 == 0;
+    for (int s0 = 0; s0 < ns; s0 += 32768) {  // grid.y ends at 65535
+        const int n = std::min(ns - s0, 32768);
+        const long long work = (vec ? N / 2 : N) + kThreads - 1;
+        const dim3 g((unsigned)std::min<long long>(work / kThreads, std::max(1, 148 * 16 / n)), (unsigned)n);
+        double* x = X + (long long)s0 * ldx;
+        const double *u = W1 + (long long)s0 * ldw, *v = W2 + (long long)s0 * ldw;
+        if (vec) k_td_update2<true><<<g, kThreads, 0, st>>>(N, x, ldx, u, v, ldw, a1, b1, a2);
+        else k_td_update2<false><<<g, kThreads, 0, st>>>(N, x, ldx, u, v, ldw, a1, b1, a2);
     }
 }
 
@@ -448,22 +473,17 @@ int qg_td_taylor4_z(qg_hamiltonian h, int ns, double dt, double* X, long long ld
     double* W2 = W1 + (size_t)ns * ldw;
     QG_TRY(h->coef.reserve(qg::nonlocal_scratch(h, 1, ns, true) * sizeof(double)));
     double* coef = h->coef.as<double>();
-    const int g = qg::grid_for((long long)ns * N);
     const double c2 = dt * dt / 2.0;
     const double c3 = c2 * dt / 3.0;
     const double c4 = c3 * dt / 4.0;
-    // x += -i dt H x
+    // x += -i dt H x, x += -(dt^2/2) H^2 x
     QG_TRY(qg::apply_hamiltonian_z<double>(h, ns, X, ldx, W1, ldw, coef, st));
-    qg::k_td_update<false><<<g, qg::kThreads, 0, st>>>(ns, N, X, ldx, W1, ldw, dt, -dt);
-    // x += -(dt^2/2) H^2 x
     QG_TRY(qg::apply_hamiltonian_z<double>(h, ns, W1, ldw, W2, ldw, coef, st));
-    qg::k_td_update<true><<<g, qg::kThreads, 0, st>>>(ns, N, X, ldx, W2, ldw, -c2, 0.0);
-    // x += i (dt^3/6) H^3 x
+    qg::launch_td_update2(ns, N, X, ldx, W1, W2, ldw, dt, -dt, -c2, st);
+    // x += i (dt^3/6) H^3 x, x += (dt^4/24) H^4 x
     QG_TRY(qg::apply_hamiltonian_z<double>(h, ns, W2, ldw, W1, ldw, coef, st));
-    qg::k_td_update<false><<<g, qg::kThreads, 0, st>>>(ns, N, X, ldx, W1, ldw, -c3, c3);
-    // x += (dt^4/24) H^4 x
     QG_TRY(qg::apply_hamiltonian_z<double>(h, ns, W1, ldw, W2, ldw, coef, st));
-    qg::k_td_update<true><<<g, qg::kThreads, 0, st>>>(ns, N, X, ldx, W2, ldw, c4, 0.0);
+    qg::launch_td_update2(ns, N, X, ldx, W1, W2, ldw, -c3, c3, c4, st);
     QG_CUDA_TRY(cudaGetLastError());
     return QG_OK;
 }
