@@ -1150,6 +1150,7 @@ int run_lobpcg_zk(qg_hamiltonian h, const qg_lobpcg_options* opt, int nk, const 
         QG_TRY(s.work.reserve((size_t)std::max(s.lwork, 1) * sizeof(cuDoubleComplex)));
     }
     QG_TRY(h->coef.reserve(qg::nonlocal_scratch(h, nk, nb, true) * sizeof(double)));
+    if (2 * nb <= qg::kGramTsMax) QG_TRY(s.gts.reserve(qg::gram_ts_scratch_doubles(N, nk, true) * sizeof(double)));
     // pencils of up to kSmallHegMax rows: all k-points' Hermitian pencils in one launch
     // of the one-block Jacobi solver (small_eig.cu), cuSOLVER's zhegvd per k-point
     // otherwise and for any pencil the Jacobi solver rejects
@@ -1178,21 +1179,25 @@ int run_lobpcg_zk(qg_hamiltonian h, const qg_lobpcg_options* opt, int nk, const 
         return qg::apply_hamiltonian_zk(h, nk, kv, nb, in, s.L, (long long)nb * s.L, out, s.L, (long long)nb * s.L,
                                         h->coef.as<double>(), st);
     };
-    // C_k (block (bi, bj) of the k-th pencil, ldc g) = dV * A_k^T B_k, one DGEMM per k-point:
-    // cuBLAS's strided-batched DGEMM at these shapes (2nb x 2nb, K = N) returned Gram
-    // matrices noticeably less accurate than its plain DGEMM (8 k-points: 208 rank-revealing
-    // restarts and 95 iterations instead of 11 and 73), so the batch is a loop of DGEMMs
-    auto gram_block = [&](const double* A, const double* B, double* C, int g) -> int {
-        const double zero = 0.0;
-        for (int k = 0; k < nk; ++k)
-            QG_BLAS_TRY(cublasDgemm(s.blas, CUBLAS_OP_T, CUBLAS_OP_N, 2 * nb, 2 * nb, (int)N, &s.dV, A + k * kstride,
-                                    (int)N, B + k * kstride, (int)N, &zero, C + k * gsz, g));
-        return QG_OK;
-    };
+    // Ca_k = dV W_k^T AW_k and Cb_k = dV W_k^T W_k (block (bi, bj) of the k-th pencil, ldc g): all
+    // k-points and both products in one split-K launch up to 64 columns, one DGEMM per k-point and
+    // product above (64000 x 32, 8 k-points: 0.09 ms against 0.32 for the 16 DGEMMs; cuBLAS's strided-batched DGEMM at these
+    // shapes returned Gram matrices noticeably less accurate than its plain DGEMM: 208
+    // rank-revealing restarts and 95 iterations instead of 11 and 73)
     auto gram_pair = [&](const double* Wi, const double* AWj, const double* Wj, double* Ca_, double* Cb_,
                          int g) -> int {
-        QG_TRY(gram_block(Wi, AWj, Ca_, g));
-        return gram_block(Wi, Wj, Cb_, g);
+        if (2 * nb <= qg::kGramTsMax)
+            return qg::gram_ts(Wi, N, kstride, AWj, Wj, N, kstride, N, 2 * nb, 2 * nb, s.dV, Ca_, Cb_, g, (long long)gsz,
+                               nk, s.gts.as<double>(), st);
+        const double zero = 0.0;
+        for (int k = 0; k < nk; ++k) {
+            const double* A = Wi + k * kstride;
+            QG_BLAS_TRY(cublasDgemm(s.blas, CUBLAS_OP_T, CUBLAS_OP_N, 2 * nb, 2 * nb, (int)N, &s.dV, A, (int)N,
+                                    AWj + k * kstride, (int)N, &zero, Ca_ + k * gsz, g));
+            QG_BLAS_TRY(cublasDgemm(s.blas, CUBLAS_OP_T, CUBLAS_OP_N, 2 * nb, 2 * nb, (int)N, &s.dV, A, (int)N,
+                                    Wj + k * kstride, (int)N, &zero, Cb_ + k * gsz, g));
+        }
+        return QG_OK;
     };
     // C_k (N x 2nb) = A_k (N x 2nb) * Z_k (rows off.., ldz) + beta C_k, batched over k
     auto rot_block = [&](const double* A, const double* Z, int ldz, double* C, double beta) -> int {
