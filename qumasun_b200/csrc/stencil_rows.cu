@@ -100,6 +100,13 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_stencil_rows(const HamArgs<
     constexpr int PX = 16 / sizeof(T);
     constexpr int R = rows_radius<ORDER>();
     constexpr int Q = 2 * R + 1;
+    // FP64: the windows rotate by renaming over Q unrolled steps. FP32 has twice the points per step
+    // and lost a third of its issue slots to instruction fetches on that code: three steps, then the
+    // windows move down, and the wait for plane z + R goes behind the loads that do not need it (256
+    // states of 80^3: 0.49 ms rotating, 0.40 so; FP64 0.552 rotating, 0.555 so).
+    constexpr bool kRotate = sizeof(T) == 8;
+    constexpr int U = kRotate ? Q : 3, kSlots = kRotate ? Q : 2 * R + U;
+    auto sl = [](int d) { return kRotate ? d % Q : d; };
     constexpr int NV = (R + PX - 1) / PX;
     using VV = R16<T>;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -159,8 +166,8 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_stencil_rows(const HamArgs<
             const int ze = min(nz, zs + wg.zslab);
             const long long col = (long long)iy0 * nx + ix0;
 
-            // z-windows of both rows: plane z - R + d in slot (k + d) % Q at unrolled step k
-            T q0[Q][PX], q1[Q][PX];
+            // z-windows of both rows: plane z - R + d in slot sl(k + d) at unrolled step k
+            T q0[kSlots][PX], q1[kSlots][PX];
             int j = pos % nst;
             uint32_t ph = (uint32_t)(pos / nst) & 1u;
             bool w = true;
@@ -194,16 +201,20 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_stencil_rows(const HamArgs<
             }
             for (int z = zs; z < ze && !bad;) {
 #pragma unroll
-                for (int k = 0; k < Q; ++k) {
+                for (int k = 0; k < U; ++k) {
                     if (z >= ze) break;
-                    const bool ok = mbar_wait(&full[jp], php);
-                    if (__any_sync(wmask, !ok)) {
+                    const int cs = sl(k + R);  // centre slot (plane z)
+                    auto next_plane = [&] {  // plane z + R
+                        const bool ok = mbar_wait(&full[jp], php);
+                        if (__any_sync(wmask, !ok)) return false;
+                        VV::ld(q0[sl(k + 2 * R)], ringp + jp * stage_elems + cb0);
+                        VV::ld(q1[sl(k + 2 * R)], ringp + jp * stage_elems + cb0 + nx);
+                        return true;
+                    };
+                    if (kRotate && !next_plane()) {
                         bad = true;
                         break;
                     }
-                    const int cs = (k + R) % Q;  // centre slot (plane z)
-                    VV::ld(q0[(k + 2 * R) % Q], ringp + jp * stage_elems + cb0);
-                    VV::ld(q1[(k + 2 * R) % Q], ringp + jp * stage_elems + cb0 + nx);
                     const T* st = ringp + jz * stage_elems;
                     // rows ly0 - R .. ly0 - 1 and ly0 + 2 .. ly0 + 1 + R (shared by both rows)
                     T ya[R][PX], yb[R][PX];
@@ -226,6 +237,10 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_stencil_rows(const HamArgs<
                             VV::ldg(vn0, vcol + (long long)(z + 1) * plane);
                             VV::ldg(vn1, vcol + (long long)(z + 1) * plane + nx);
                         }
+                    }
+                    if (!kRotate && !next_plane()) {
+                        bad = true;
+                        break;
                     }
                     T out0[PX], out1[PX];
 #pragma unroll
@@ -251,13 +266,13 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_stencil_rows(const HamArgs<
                                 if (row == 0) {
                                     ym[d - 1] = ya[d - 1][e];
                                     yp[d - 1] = d == 1 ? q1[cs][e] : yb[d - 2][e];
-                                    zm[d - 1] = q0[(k + R - d) % Q][e];
-                                    zp[d - 1] = q0[(k + R + d) % Q][e];
+                                    zm[d - 1] = q0[sl(k + R - d)][e];
+                                    zp[d - 1] = q0[sl(k + R + d)][e];
                                 } else {
                                     ym[d - 1] = d == 1 ? q0[cs][e] : ya[d - 2][e];
                                     yp[d - 1] = yb[d - 1][e];
-                                    zm[d - 1] = q1[(k + R - d) % Q][e];
-                                    zp[d - 1] = q1[(k + R + d) % Q][e];
+                                    zm[d - 1] = q1[sl(k + R - d)][e];
+                                    zp[d - 1] = q1[sl(k + R + d)][e];
                                 }
                             }
                             const T cval = row ? q1[cs][e] : q0[cs][e];
@@ -282,6 +297,15 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_stencil_rows(const HamArgs<
                     ++z;
                     if (++jz == nst) jz = 0;
                     if (++jp == nst) { jp = 0; php ^= 1u; }
+                }
+                if constexpr (!kRotate) {
+#pragma unroll
+                    for (int d = 0; d < 2 * R; ++d)
+#pragma unroll
+                        for (int e = 0; e < PX; ++e) {
+                            q0[d][e] = q0[d + U][e];
+                            q1[d][e] = q1[d + U][e];
+                        }
                 }
             }
             if (bad) break;
