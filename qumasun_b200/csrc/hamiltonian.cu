@@ -440,6 +440,11 @@ template <> struct Vec16<float> {
     }
 };
 
+// Two neighbouring points.
+template <typename T> struct Pair2;
+template <> struct Pair2<double> { using type = double2; };
+template <> struct Pair2<float> { using type = float2; };
+
 // Nonlocal scatter over all states, one thread per grid point. The point's first
 // KMAX entries (their coefficient rows and NCH table values) stay in registers for
 // all state groups; for each group of SG states every entry adds
@@ -532,9 +537,104 @@ static int launch_scatter_all_nch(const DevProjectors& pj, T* HX, long long ldhx
     return QG_OK;
 }
 
+// The scatter with two neighbouring grid points (2 i, 2 i + 1) per thread: an entry holds the values of one
+// atom at both points (zero where only one lies in the sphere), so a coefficient vector read from
+// L1 serves both. k_scatter_all spends 80 % of its L1 bandwidth on those vectors and 75 % of the
+// peak in all: 0.52 ms for 256 states of 80^3, 3.49 ms for 528 of 120^3, FP32 0.31 ms; pairs
+// 0.44, 3.11 and 0.23 ms (a read and a write of H psi: 0.31, 2.2 and 0.16). Groups of 4 FP64 states: 8 spill (0.62 ms). blockIdx.y splits the states where the
+// pairs alone are few waves of blocks. A NaN or Inf coefficient reaches the other point of a pair (0 * NaN).
+template <typename T, int SG, int NCH, int KMAX>
+__global__ void __launch_bounds__(256, 2) k_scatter_pairs(T* __restrict__ HX, long long ldhx, int ns, long long npairs,
+                                                          const int* __restrict__ row, const int* __restrict__ ent_atom,
+                                                          const T* __restrict__ ent_val, const T* __restrict__ coef,
+                                                          long long ldc) {
+    using V = typename Vec16<T>::type;
+    using P = typename Pair2<T>::type;
+    constexpr int VN = Vec16<T>::n;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= npairs) return;
+    const int e0 = row[i], ne = row[i + 1] - e0;
+    if (ne == 0) return;
+    const P* ev = reinterpret_cast<const P*>(ent_val);
+    int cb[KMAX];  // first coefficient row of the entry's atom
+    P v[KMAX][NCH];
+#pragma unroll
+    for (int k = 0; k < KMAX; ++k) {
+        cb[k] = 0;
+        if (k < ne) {
+            cb[k] = __ldg(&ent_atom[e0 + k]) * NCH;
+#pragma unroll
+            for (int c = 0; c < NCH; ++c) v[k][c] = __ldg(&ev[(long long)(e0 + k) * NCH + c]);
+        }
+    }
+    const int per = ((ns + gridDim.y - 1) / gridDim.y + SG - 1) / SG * SG;
+    const int se = min(ns, (int)(blockIdx.y + 1) * per);
+    for (int s0 = blockIdx.y * per; s0 < se; s0 += SG) {
+        const int gn = min(SG, se - s0);
+        P* h0 = reinterpret_cast<P*>(HX + (long long)s0 * ldhx) + i;
+        const long long step = ldhx / 2;
+        P h[SG];
+#pragma unroll
+        for (int s = 0; s < SG; ++s)
+            if (s < gn) h[s] = h0[s * step];
+        T a0[SG], a1[SG];
+#pragma unroll
+        for (int s = 0; s < SG; ++s) a0[s] = a1[s] = T(0);
+        auto add = [&](int base, int c, const P& val) {
+            const V* cp = reinterpret_cast<const V*>(coef + (long long)(base + c) * ldc + s0);
+#pragma unroll
+            for (int j = 0; j < SG / VN; ++j) {
+                const V w = __ldg(cp + j);
+#pragma unroll
+                for (int q = 0; q < VN; ++q) {
+                    a0[j * VN + q] += val.x * Vec16<T>::at(w, q);
+                    a1[j * VN + q] += val.y * Vec16<T>::at(w, q);
+                }
+            }
+        };
+#pragma unroll
+        for (int k = 0; k < KMAX; ++k)
+            if (k < ne)
+#pragma unroll
+                for (int c = 0; c < NCH; ++c) add(cb[k], c, v[k][c]);
+        for (int e = e0 + KMAX; e < e0 + ne; ++e) {
+            const int base = __ldg(&ent_atom[e]) * NCH;
+#pragma unroll
+            for (int c = 0; c < NCH; ++c) add(base, c, __ldg(&ev[(long long)e * NCH + c]));
+        }
+#pragma unroll
+        for (int s = 0; s < SG; ++s)
+            if (s < gn) {
+                h[s].x += a0[s];
+                h[s].y += a1[s];
+                h0[s * step] = h[s];
+            }
+    }
+}
+
+// Pairs where the rows can be read two points at a time and the pairs are many enough to fill the SMs
+// (one wave of two blocks per SM).
+template <typename T>
+static bool scatter_by_pairs(const DevProjectors& pj, const T* HX, long long ldhx, long long N) {
+    return pj.pair_row && N % 2 == 0 && ldhx % 2 == 0 && (uintptr_t)HX % (2 * sizeof(T)) == 0 &&
+           N / 2 >= 2LL * 148 * 256;
+}
+
 template <typename T>
 static int launch_scatter_all(const DevProjectors& pj, T* HX, long long ldhx, int ns, long long N, const T* coef,
                               long long ldc, int forced_sg, cudaStream_t st) {
+    if (scatter_by_pairs<T>(pj, HX, ldhx, N)) {
+        const T* ev;
+        if constexpr (sizeof(T) == 8) ev = reinterpret_cast<const T*>(pj.pair_val_d);
+        else ev = reinterpret_cast<const T*>(pj.pair_val_f);
+        const int blocks = (int)((N / 2 + 255) / 256);
+        // at least eight waves of two blocks per SM, 32 states or more per block
+        const int split = std::max(1, std::min((ns + 31) / 32, (8 * 2 * 148 + blocks - 1) / blocks));
+        const int sg = forced_sg ? forced_sg : (sizeof(T) == 8 ? 4 : 8);
+        auto kern = sg == 4 ? k_scatter_pairs<T, 4, 4, 3> : k_scatter_pairs<T, 8, 4, 3>;
+        kern<<<dim3(blocks, split), 256, 0, st>>>(HX, ldhx, ns, N / 2, pj.pair_row, pj.pair_atom, ev, coef, ldc);
+        return QG_OK;
+    }
     const int sg = forced_sg == 4 ? 4 : 8;
     switch (pj.nch) {
         case 4: return launch_scatter_all_nch<T, 4>(pj, HX, ldhx, ns, N, coef, ldc, sg, st);
@@ -579,7 +679,8 @@ size_t coef_scratch_elems(qg_hamiltonian h, int ns) {
 // else the two-row ring kernel -- FP64 with V in the ring (4), FP32 with V from global
 // memory (5) -- measured on the 80^3 cell, 256 states (whole apply, order 2/4/6/8):
 // FP64 4: 1.46/1.52/1.52/1.55 ms, 5: 1.58/1.59/1.59/1.59, one-plane (2): 1.52/1.75/1.77/1.77;
-// FP32 5: 0.87/1.03/1.03/1.10, 4: 1.00/1.06/1.04/1.11, 2: 0.91/1.11/1.10/1.12;
+// FP32 5: 0.87/1.03/1.03/1.10, 4: 1.00/1.06/1.04/1.11, 2: 0.91/1.11/1.10/1.12 (order 8 of 5 is 0.95
+// since its windows move; the projection and the scatter have changed too, for all alike);
 // then the other ring kernels, else (1) the register-window kernel, which takes any
 // shape. All ring kernels give the same bits.
 template <typename T>
@@ -718,6 +819,7 @@ void free_projectors(DevProjectors& pj) {
     cudaFree(pj.atom_off); cudaFree(pj.pt_g); cudaFree(pj.tab_d); cudaFree(pj.tab_f);
     cudaFree(pj.ch_scale); cudaFree(pj.ch_dv); cudaFree(pj.ch_E); cudaFree(pj.row); cudaFree(pj.ent_atom); cudaFree(pj.ent_val_d);
     cudaFree(pj.ent_val_f);
+    cudaFree(pj.pair_row); cudaFree(pj.pair_atom); cudaFree(pj.pair_val_d); cudaFree(pj.pair_val_f);
     qg::free_bricks(pj.bricks);
     pj = DevProjectors();
 }
@@ -818,6 +920,32 @@ int build_projectors(qg_hamiltonian h, const qg_hamiltonian_desc* d) {
         }
     std::vector<float> ent_val_f(ent_val.begin(), ent_val.end());
 
+    // the entries of points 2 i and 2 i + 1 merged by atom (an atom that covers a point through several
+    // images has an entry for each): pair_val[e * nch + ch] = {value at 2 i, value at 2 i + 1}
+    std::vector<int> pair_row, pair_atom;
+    std::vector<double> pair_val;
+    if (nch == 4 && N % 2 == 0) {
+        pair_row.reserve(N / 2 + 1);
+        pair_row.push_back(0);
+        for (long long i = 0; i < N / 2; ++i) {
+            int e[2] = {row[2 * i], row[2 * i + 1]};
+            const int end[2] = {row[2 * i + 1], row[2 * i + 2]};
+            while (e[0] < end[0] || e[1] < end[1]) {
+                int a = na;
+                for (int q = 0; q < 2; ++q)
+                    if (e[q] < end[q]) a = std::min(a, ent_atom[e[q]]);
+                pair_atom.push_back(a);
+                const double* src[2] = {nullptr, nullptr};
+                for (int q = 0; q < 2; ++q)
+                    if (e[q] < end[q] && ent_atom[e[q]] == a) src[q] = &ent_val[(size_t)nch * e[q]++];
+                for (int ch = 0; ch < nch; ++ch)
+                    for (int q = 0; q < 2; ++q) pair_val.push_back(src[q] ? src[q][ch] : 0.0);
+            }
+            pair_row.push_back((int)pair_atom.size());
+        }
+    }
+    std::vector<float> pair_val_f(pair_val.begin(), pair_val.end());
+
     DevProjectors& pj = h->pj;
     pj.na = na; pj.nch = nch; pj.npts = npts; pj.nent = npts;
     pj.max_atom_pts = 0;
@@ -833,6 +961,10 @@ int build_projectors(qg_hamiltonian h, const qg_hamiltonian_desc* d) {
     QG_TRY(upload(&pj.ent_atom, ent_atom));
     QG_TRY(upload(&pj.ent_val_d, ent_val));
     QG_TRY(upload(&pj.ent_val_f, ent_val_f));
+    QG_TRY(upload(&pj.pair_row, pair_row));
+    QG_TRY(upload(&pj.pair_atom, pair_atom));
+    QG_TRY(upload(&pj.pair_val_d, pair_val));
+    QG_TRY(upload(&pj.pair_val_f, pair_val_f));
     return qg::build_bricks(h, atom_off, pt_u, tabs);
 }
 

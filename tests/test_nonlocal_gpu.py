@@ -106,6 +106,33 @@ def test_kpoint_projection_and_scatter_match_oracle(cuda_ctx, name, ns, dtype):
     H.close()
 
 
+@pytest.mark.parametrize("f64", [True, False], ids=["f64", "f32"])
+@pytest.mark.parametrize("ns", [1, 5, 37])
+@pytest.mark.parametrize("kw", [dict(reps=(1, 1, 3), grid=(40, 38, 100), displacement=0.1, seed=3),
+                                dict(grid=(54, 54, 54), a0=4.4)], ids=["ragged", "wrap"])
+def test_scatter_by_pairs_matches_oracle(cuda_ctx, kw, ns, f64):
+    """Grids large enough for the scatter of two points per thread; rows of odd length go point by
+    point (the same entries in the same order)."""
+    import torch
+    from qumasun_b200 import Hamiltonian
+    cell = build_cell(**kw)
+    X = initial_states(ns, cell.N, seed=ns)
+    H = Hamiltonian(cuda_ctx, cell)
+    Xd = torch.from_numpy(X).cuda().to(torch.float64 if f64 else torch.float32)
+    pairs = H.apply(Xd)
+    assert rel(pairs.double().cpu().numpy(), O.hamiltonian_apply(cell, X)) < (1e-12 if f64 else 2e-6)
+    for sg in (4, 8):
+        H.set_nonlocal_blocking(0, sg, 0)
+        assert torch.equal(H.apply(Xd), pairs)
+    H.set_nonlocal_blocking(0, 0, 0)
+    hb, hv = padded(torch.zeros_like(Xd), 1, 1)
+    torch.cuda.synchronize()
+    H.apply_device(ns, Xd.data_ptr(), hv.data_ptr(), cell.N, cell.N + 1, "f64" if f64 else "f32")
+    cuda_ctx.synchronize()
+    assert rel(hv.double().cpu().numpy(), pairs.double().cpu().numpy()) < (1e-14 if f64 else 1e-6)
+    H.close()
+
+
 @pytest.mark.parametrize("kw", [dict(grid=(13, 11, 9)), dict(grid=(27, 17, 15), displacement=0.05, seed=1)],
                          ids=["8-atoms-tiny", "8-atoms"])
 @pytest.mark.parametrize("f64", [True, False], ids=["f64", "f32"])
