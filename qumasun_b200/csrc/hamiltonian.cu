@@ -94,6 +94,7 @@ __global__ void __launch_bounds__(1024) k_hamiltonian(const HamArgs<T> a) {
     constexpr int Q = 2 * R + 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* sm = reinterpret_cast<T*>(smem_raw);
+    allow_next();
 
     const int nx = a.nx, ny = a.ny, nz = a.nz, ty = a.ty;
     const int W = nx + 2 * R;
@@ -178,6 +179,7 @@ __global__ void __launch_bounds__(1024) k_hamiltonian(const HamArgs<T> a) {
             }
         }
     }
+    wait_previous();
 }
 
 // Gather-contraction of the projectors. `chunks` blocks serve one (atom, group of
@@ -220,6 +222,7 @@ __global__ void __launch_bounds__(kProjThreads) k_project(const T* __restrict__ 
                                                  const T* __restrict__ tab, long long npts,
                                                  const double* __restrict__ ch_scale,
                                                  T* __restrict__ coef, long long ldc, int chunks) {
+    allow_next();
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank();
     const int atom = blockIdx.x / chunks;
@@ -457,7 +460,7 @@ __global__ void __launch_bounds__(256, SG <= 4 ? 3 : 2) k_scatter_all(T* __restr
                                                      const int* __restrict__ row,
                                                      const int* __restrict__ ent_atom,
                                                      const T* __restrict__ ent_val,
-                                                     const T* __restrict__ coef, long long ldc) {
+                                                     const T* coef, long long ldc) {
     using V = typename Vec16<T>::type;
     constexpr int VN = Vec16<T>::n;
     static_assert(SG % VN == 0, "state group must be whole vectors");
@@ -478,6 +481,7 @@ __global__ void __launch_bounds__(256, SG <= 4 ? 3 : 2) k_scatter_all(T* __restr
             for (int c = 0; c < NCH; ++c) v[k][c] = __ldg(&ent_val[(long long)(e0 + k) * NCH + c]);
         }
     }
+    wait_previous();  // coef through plain loads: the read-only path may be read ahead of this
     for (int s0 = 0; s0 < ns; s0 += SG) {
         // the group's H psi values load first, so their latency overlaps the sums
         const int gn = min(SG, ns - s0);
@@ -495,7 +499,7 @@ __global__ void __launch_bounds__(256, SG <= 4 ? 3 : 2) k_scatter_all(T* __restr
                     const V* cp = reinterpret_cast<const V*>(coef + (long long)(cb[k] + c) * ldc + s0);
 #pragma unroll
                     for (int j = 0; j < SG / VN; ++j) {
-                        const V w = __ldg(cp + j);
+                        const V w = cp[j];
 #pragma unroll
                         for (int i = 0; i < VN; ++i) acc[j * VN + i] += v[k][c] * Vec16<T>::at(w, i);
                     }
@@ -510,7 +514,7 @@ __global__ void __launch_bounds__(256, SG <= 4 ? 3 : 2) k_scatter_all(T* __restr
                 const V* cp = reinterpret_cast<const V*>(ce + (long long)c * ldc + s0);
 #pragma unroll
                 for (int j = 0; j < SG / VN; ++j) {
-                    const V w = __ldg(cp + j);
+                    const V w = cp[j];
 #pragma unroll
                     for (int i = 0; i < VN; ++i) acc[j * VN + i] += vc * Vec16<T>::at(w, i);
                 }
@@ -524,16 +528,18 @@ __global__ void __launch_bounds__(256, SG <= 4 ? 3 : 2) k_scatter_all(T* __restr
 
 template <typename T, int NCH>
 static int launch_scatter_all_nch(const DevProjectors& pj, T* HX, long long ldhx, int ns, long long N,
-                                  const T* coef, long long ldc, int sg, cudaStream_t st) {
+                                  const T* coef, long long ldc, int sg, bool early, cudaStream_t st) {
     constexpr int KMAX = NCH <= 4 ? 3 : (NCH == 8 ? 2 : 1);
     const T* ev;
     if constexpr (sizeof(T) == 8) ev = reinterpret_cast<const T*>(pj.ent_val_d);
     else ev = reinterpret_cast<const T*>(pj.ent_val_f);
     const unsigned grid = (unsigned)((N + 255) / 256);
     if (sg == 4)
-        k_scatter_all<T, 4, NCH, KMAX><<<grid, 256, 0, st>>>(HX, ldhx, ns, N, pj.row, pj.ent_atom, ev, coef, ldc);
+        QG_CUDA_TRY(launch_kernel(early, k_scatter_all<T, 4, NCH, KMAX>, dim3(grid), dim3(256), 0, st, HX, ldhx, ns, N, pj.row, pj.ent_atom,
+                                  ev, coef, ldc));
     else
-        k_scatter_all<T, 8, NCH, KMAX><<<grid, 256, 0, st>>>(HX, ldhx, ns, N, pj.row, pj.ent_atom, ev, coef, ldc);
+        QG_CUDA_TRY(launch_kernel(early, k_scatter_all<T, 8, NCH, KMAX>, dim3(grid), dim3(256), 0, st, HX, ldhx, ns, N, pj.row, pj.ent_atom,
+                                  ev, coef, ldc));
     return QG_OK;
 }
 
@@ -546,7 +552,7 @@ static int launch_scatter_all_nch(const DevProjectors& pj, T* HX, long long ldhx
 template <typename T, int SG, int NCH, int KMAX>
 __global__ void __launch_bounds__(256, 2) k_scatter_pairs(T* __restrict__ HX, long long ldhx, int ns, long long npairs,
                                                           const int* __restrict__ row, const int* __restrict__ ent_atom,
-                                                          const T* __restrict__ ent_val, const T* __restrict__ coef,
+                                                          const T* __restrict__ ent_val, const T* coef,
                                                           long long ldc) {
     using V = typename Vec16<T>::type;
     using P = typename Pair2<T>::type;
@@ -567,6 +573,7 @@ __global__ void __launch_bounds__(256, 2) k_scatter_pairs(T* __restrict__ HX, lo
             for (int c = 0; c < NCH; ++c) v[k][c] = __ldg(&ev[(long long)(e0 + k) * NCH + c]);
         }
     }
+    wait_previous();
     const int per = ((ns + gridDim.y - 1) / gridDim.y + SG - 1) / SG * SG;
     const int se = min(ns, (int)(blockIdx.y + 1) * per);
     for (int s0 = blockIdx.y * per; s0 < se; s0 += SG) {
@@ -584,7 +591,7 @@ __global__ void __launch_bounds__(256, 2) k_scatter_pairs(T* __restrict__ HX, lo
             const V* cp = reinterpret_cast<const V*>(coef + (long long)(base + c) * ldc + s0);
 #pragma unroll
             for (int j = 0; j < SG / VN; ++j) {
-                const V w = __ldg(cp + j);
+                const V w = cp[j];
 #pragma unroll
                 for (int q = 0; q < VN; ++q) {
                     a0[j * VN + q] += val.x * Vec16<T>::at(w, q);
@@ -622,7 +629,7 @@ static bool scatter_by_pairs(const DevProjectors& pj, const T* HX, long long ldh
 
 template <typename T>
 static int launch_scatter_all(const DevProjectors& pj, T* HX, long long ldhx, int ns, long long N, const T* coef,
-                              long long ldc, int forced_sg, cudaStream_t st) {
+                              long long ldc, int forced_sg, bool early, cudaStream_t st) {
     if (scatter_by_pairs<T>(pj, HX, ldhx, N)) {
         const T* ev;
         if constexpr (sizeof(T) == 8) ev = reinterpret_cast<const T*>(pj.pair_val_d);
@@ -632,14 +639,15 @@ static int launch_scatter_all(const DevProjectors& pj, T* HX, long long ldhx, in
         const int split = std::max(1, std::min((ns + 31) / 32, (8 * 2 * 148 + blocks - 1) / blocks));
         const int sg = forced_sg ? forced_sg : (sizeof(T) == 8 ? 4 : 8);
         auto kern = sg == 4 ? k_scatter_pairs<T, 4, 4, 3> : k_scatter_pairs<T, 8, 4, 3>;
-        kern<<<dim3(blocks, split), 256, 0, st>>>(HX, ldhx, ns, N / 2, pj.pair_row, pj.pair_atom, ev, coef, ldc);
+        QG_CUDA_TRY(launch_kernel(early, kern, dim3(blocks, split), dim3(256), 0, st, HX, ldhx, ns, N / 2, pj.pair_row,
+                                  pj.pair_atom, ev, coef, ldc));
         return QG_OK;
     }
     const int sg = forced_sg == 4 ? 4 : 8;
     switch (pj.nch) {
-        case 4: return launch_scatter_all_nch<T, 4>(pj, HX, ldhx, ns, N, coef, ldc, sg, st);
-        case 8: return launch_scatter_all_nch<T, 8>(pj, HX, ldhx, ns, N, coef, ldc, sg, st);
-        case 16: return launch_scatter_all_nch<T, 16>(pj, HX, ldhx, ns, N, coef, ldc, sg, st);
+        case 4: return launch_scatter_all_nch<T, 4>(pj, HX, ldhx, ns, N, coef, ldc, sg, early, st);
+        case 8: return launch_scatter_all_nch<T, 8>(pj, HX, ldhx, ns, N, coef, ldc, sg, early, st);
+        case 16: return launch_scatter_all_nch<T, 16>(pj, HX, ldhx, ns, N, coef, ldc, sg, early, st);
         default: return QG_ERR_UNSUPPORTED;
     }
 }
@@ -665,7 +673,7 @@ static int launch_stencil(const HamArgs<T>& a, int nz, cudaStream_t st) {
             return QG_ERR_UNSUPPORTED;
     }
     dim3 grid(tiles, sgroups, nslab);
-    kern<<<grid, a.nx * a.ty, smem, st>>>(b);
+    QG_CUDA_TRY(launch_kernel(a.early, kern, grid, dim3(a.nx * a.ty), smem, st, b));
     return QG_OK;
 }
 
@@ -757,32 +765,39 @@ int apply_hamiltonian(qg_hamiltonian h, int ns, const T* X, long long ldx, T* HX
     const int variant = ring_stencil_variant<T>(h, a);
     T* coef = static_cast<T*>(scratch);
     if (pt) pt->mark(nonlocal ? 0 : 1, st);
+    auto stencil = [&](bool early) -> int {
+        a.early = early;
+        if (variant == 3) return launch_stencil_pair<T>(a, h->order, st);
+        if (variant == 4) return launch_stencil_rows<T>(a, h->order, st, true);
+        if (variant == 5) return launch_stencil_rows<T>(a, h->order, st, false);
+        if (variant == 2) return launch_stencil_tma<T>(a, h->order, st);
+        if (h->order == 2) return launch_stencil<T, 2>(a, h->nz, st);
+        if (h->order == 4) return launch_stencil<T, 4>(a, h->nz, st);
+        if (h->order == 6) return launch_stencil<T, 6>(a, h->nz, st);
+        return launch_stencil<T, 8>(a, h->nz, st);
+    };
+    const bool together = nonlocal && !pt;  // events between the kernels would order them
+    bool done = false;                      // the stencil is launched
     if (nonlocal) {
         // FP32 states, a forced split of the atoms and the no-allocation entry point go atom by atom
         bool bricks = !atom_major && h->proj_parts == 0 && bricks_for_real(pj);
         if constexpr (sizeof(T) == 8) {
-            if (bricks)
+            if (bricks) {
                 QG_TRY(brick_project<T>(h, 1, ns, false, X, ldx, 0, nullptr, pj.ch_scale, coef,
-                                        coef + coef_elems(h, 1, ns, false), st));
+                                        coef + coef_elems(h, 1, ns, false), st,
+                                        together ? std::function<int(bool)>(stencil) : std::function<int(bool)>()));
+                done = together;
+            }
         } else {
             bricks = false;
         }
         if (!bricks) QG_TRY(launch_project<T>(pj, ns, X, ldx, coef, coef_ld(ns), h->proj_sb, h->proj_parts, st));
         if (pt) pt->mark(1, st);
     }
-    int rc;
-    if (variant == 3) rc = launch_stencil_pair<T>(a, h->order, st);
-    else if (variant == 4) rc = launch_stencil_rows<T>(a, h->order, st, true);
-    else if (variant == 5) rc = launch_stencil_rows<T>(a, h->order, st, false);
-    else if (variant == 2) rc = launch_stencil_tma<T>(a, h->order, st);
-    else if (h->order == 2) rc = launch_stencil<T, 2>(a, h->nz, st);
-    else if (h->order == 4) rc = launch_stencil<T, 4>(a, h->nz, st);
-    else if (h->order == 6) rc = launch_stencil<T, 6>(a, h->nz, st);
-    else rc = launch_stencil<T, 8>(a, h->nz, st);
-    QG_TRY(rc);
+    if (!done) QG_TRY(stencil(together));
     if (nonlocal) {
         if (pt) pt->mark(2, st);
-        QG_TRY(launch_scatter_all<T>(pj, HX, ldhx, ns, N, coef, coef_ld(ns), h->scatter_sg, st));
+        QG_TRY(launch_scatter_all<T>(pj, HX, ldhx, ns, N, coef, coef_ld(ns), h->scatter_sg, together && small_call((long long)ns * N), st));
     }
     if (pt) pt->mark(-1, st);
     QG_CUDA_TRY(cudaGetLastError());

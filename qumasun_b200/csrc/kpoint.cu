@@ -186,25 +186,32 @@ int apply_hamiltonian_zk(qg_hamiltonian h, int nk, const double* kv, int nsk, co
     const bool nonlocal = pj.na > 0 && pj.nch > 0;
     if (pt) pt->mark(0, st);
     const double2* phase = nullptr;
+    constexpr int PX = 16 / sizeof(T);
+    const bool plain = h->stencil_variant == 1 || !stencil_kpoint_ok<T>(a, h->order) || (nk > 1 && (ldk % PX || ldkh % PX));
+    auto stencil = [&](bool early) -> int {
+        if (plain) {
+            dim3 g((unsigned)((N + 255) / 256), (unsigned)(nk * nsk));
+            switch (h->order) {
+                case 2: k_kpoint_plain<T, 2><<<g, 256, 0, st>>>(a); break;
+                case 6: k_kpoint_plain<T, 6><<<g, 256, 0, st>>>(a); break;
+                default: k_kpoint_plain<T, 8><<<g, 256, 0, st>>>(a); break;
+            }
+            return QG_OK;
+        }
+        a.early = early;
+        return launch_stencil_kpoint<T>(a, h->order, st);
+    };
+    const bool together = nonlocal && !pt;  // events between the kernels would order them
     if (nonlocal) {
         QG_TRY(ensure_phases(h, nk, kv, st, &phase));
         QG_TRY(brick_project<T>(h, nk, nsk, true, X, ldx, ldk, phase, pj.ch_scale, scratch,
-                                scratch + coef_elems(h, nk, nsk, true), st));
+                                scratch + coef_elems(h, nk, nsk, true), st,
+                                together ? std::function<int(bool)>(stencil) : std::function<int(bool)>()));
     }
     if (pt) pt->mark(1, st);
-    constexpr int PX = 16 / sizeof(T);
-    if (h->stencil_variant == 1 || !stencil_kpoint_ok<T>(a, h->order) || (nk > 1 && (ldk % PX || ldkh % PX))) {
-        dim3 g((unsigned)((N + 255) / 256), (unsigned)(nk * nsk));
-        switch (h->order) {
-            case 2: k_kpoint_plain<T, 2><<<g, 256, 0, st>>>(a); break;
-            case 6: k_kpoint_plain<T, 6><<<g, 256, 0, st>>>(a); break;
-            default: k_kpoint_plain<T, 8><<<g, 256, 0, st>>>(a); break;
-        }
-    } else {
-        QG_TRY(launch_stencil_kpoint<T>(a, h->order, st));
-    }
+    if (!together) QG_TRY(stencil(false));
     if (pt) pt->mark(2, st);
-    if (nonlocal) QG_TRY(brick_scatter_z<T>(h, nk, nsk, HX, ldhx, ldkh, phase, scratch, st));
+    if (nonlocal) QG_TRY(brick_scatter_z<T>(h, nk, nsk, HX, ldhx, ldkh, phase, scratch, together && !plain && small_call((long long)nk * nsk * N), st));
     if (pt) pt->mark(-1, st);
     QG_CUDA_TRY(cudaGetLastError());
     return QG_OK;

@@ -42,6 +42,8 @@
 #include <cstring>
 #include <unordered_map>
 
+#include "stencil_common.cuh"
+
 namespace qg {
 namespace {
 
@@ -270,16 +272,18 @@ __global__ void __launch_bounds__(kThreads, 2)
 // sums, then warp 0's lanes add the eighths in order. refs: {2 * pair + half, image}.
 template <bool CPLX>
 __global__ void __launch_bounds__(kThreads)
-    k_brick_reduce(const double* __restrict__ part, long long prow, const int* __restrict__ cg_off,
+    k_brick_reduce(const double* part, long long prow, const int* __restrict__ cg_off,
                    const int2* __restrict__ cg_ref, int ncg, int per_k, int unit0, const double2* __restrict__ phase,
                    int nphase, int img0, const double* __restrict__ scale, double* __restrict__ coef, long long rows) {
     __shared__ double sm[8][2][32];
+    allow_next();
     const int cg = blockIdx.x, u = unit0 + blockIdx.y, k = u / per_k;
     const long long lg = u - k * per_k;  // unit of the k-point
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r0 = cg_off[cg], n = cg_off[cg + 1] - r0;
     const int b0 = r0 + n * w / 8, b1 = r0 + n * (w + 1) / 8;
     const long long row = (long long)blockIdx.y * (CPLX ? 16 : 8) + (lane >> 2);
+    wait_previous();  // part through plain loads: the read-only path may be read ahead of this
     const double* p = part + row * 8 + (lane & 3);
     double re = 0.0, im = 0.0;
 #pragma unroll 4
@@ -314,7 +318,7 @@ template <typename T, bool VEC, bool ROWS, int D>
 __global__ void __launch_bounds__(kThreads, 2)
     k_brick_scatter(T* __restrict__ HX, long long ldx, long long ldk, long long xim, int ns, int per_k, int nunit,
                     const BrickGeom g, const double2* __restrict__ phase, int nphase, int img0,
-                    const double* __restrict__ coef, int ncg, long long rows) {
+                    const double* coef, int ncg, long long rows) {
     extern __shared__ __align__(16) double tb[];
     const int chunks = ROWS ? nunit : (nunit + 7) / 8;
     const int brick = blockIdx.x / chunks, ch = blockIdx.x - brick * chunks;
@@ -330,6 +334,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     const double2* ph = phase + (long long)k * nphase;
     const int row_a = ROWS ? w : 0, row_b = ROWS ? w + 1 : 8;
     using P2 = typename Pair<T>::type;
+    wait_previous();
     for (int item = g.brick_item[brick]; item < g.brick_item[brick + 1]; ++item) {
         P2 hv[D][2];
         auto fetch = [&](u64 m, int row, int b, P2 (&v)[2]) {
@@ -352,7 +357,7 @@ __global__ void __launch_bounds__(kThreads, 2)
             A[j][0] = A[j][1] = 0.0;
             if (cg >= 0) {
                 const double* c = &coef[(((long long)k * ncg + cg) * rows + lu * 16) * 4 + lane];
-                const double re = __ldg(c), im = __ldg(c + 32);
+                const double re = c[0], im = c[32];
                 const double2 p = __ldg(&ph[img0 + g.item_img[item * 8 + j]]);
                 A[j][0] = p.x * re + p.y * im;
                 A[j][1] = p.x * im - p.y * re;
@@ -451,7 +456,8 @@ int slice_units(const BrickTables& b, bool cplx, int units) {
 
 template <typename T, bool CPLX, bool VEC, bool ROWS>
 int launch_project(qg_hamiltonian h, int nk, int ns, const T* X, long long ldx, long long ldk, const double2* phase,
-                   const double* scale, double* coef, double* part, cudaStream_t st) {
+                   const double* scale, double* coef, double* part, cudaStream_t st,
+                   const std::function<int(bool)>& stencil) {
     constexpr int D = CPLX ? 4 : 8;
     const BrickTables& b = h->pj.bricks;
     const int per_k = (ns + 7) / 8, units = nk * per_k, most = slice_units(b, CPLX, units);
@@ -463,25 +469,29 @@ int launch_project(qg_hamiltonian h, int nk, int ns, const T* X, long long ldx, 
         const long long prow = (long long)nu * (CPLX ? 16 : 8);
         kern<<<(unsigned)((long long)b.nitems * (ROWS ? nu : (nu + 7) / 8)), kThreads, (size_t)b.max_tab * 512, st>>>(
             X, ldx, ldk, h->N(), ns, per_k, u0, nu, geom(h), phase, np, part, prow);
-        k_brick_reduce<CPLX><<<dim3(b.ncg, nu), kThreads, 0, st>>>(part, prow, b.cg_off, b.cg_ref, b.ncg, per_k, u0, phase,
-                                                                    np, h->nx + h->ny + h->nz, scale, coef,
-                                                                    coef_rows(ns, CPLX));
+        // one slice: the stencil runs beside the projection, and ends after it
+        const bool beside = stencil && nu == units;
+        if (beside) QG_TRY(stencil(true));
+        QG_CUDA_TRY(launch_kernel(beside && small_call((long long)nk * ns * h->N()), k_brick_reduce<CPLX>, dim3(b.ncg, nu),
+                                  dim3(kThreads), 0, st, part, prow, b.cg_off, b.cg_ref, b.ncg, per_k, u0, phase, np,
+                                  h->nx + h->ny + h->nz, scale, coef, coef_rows(ns, CPLX)));
     }
+    if (stencil && units > most) QG_TRY(stencil(false));
     QG_CUDA_TRY(cudaGetLastError());
     return QG_OK;
 }
 
 template <typename T, bool VEC, bool ROWS>
 int launch_scatter(qg_hamiltonian h, int nk, int ns, T* HX, long long ldx, long long ldk, const double2* phase,
-                   const double* coef, cudaStream_t st) {
+                   const double* coef, bool early, cudaStream_t st) {
     const BrickTables& b = h->pj.bricks;
     const int per_k = (ns + 7) / 8, units = nk * per_k;
     auto kern = k_brick_scatter<T, VEC, ROWS, 4>;
     if (allow_max_dynamic_smem(kern) != cudaSuccess) return QG_ERR_CUDA;
-    kern<<<(unsigned)((long long)b.nbricks * (ROWS ? units : (units + 7) / 8)), kThreads, (size_t)b.max_tab * 512, st>>>(
-        HX, ldx, ldk, h->N(), ns, per_k, units, geom(h), phase, phase_count(h), h->nx + h->ny + h->nz, coef, b.ncg,
-        coef_rows(ns, true));
-    QG_CUDA_TRY(cudaGetLastError());
+    QG_CUDA_TRY(launch_kernel(
+        early, kern, dim3((unsigned)((long long)b.nbricks * (ROWS ? units : (units + 7) / 8))), dim3(kThreads),
+        (size_t)b.max_tab * 512, st, HX, ldx, ldk, h->N(), ns, per_k, units, geom(h), phase, phase_count(h), h->nx + h->ny + h->nz, coef, b.ncg,
+        coef_rows(ns, true)));
     return QG_OK;
 }
 
@@ -523,16 +533,17 @@ int brick_project_launches(qg_hamiltonian h, int ns) {
 
 template <typename T>
 int brick_project(qg_hamiltonian h, int nk, int ns, bool cplx, const T* X, long long ldx, long long ldk,
-                  const double2* phase, const double* scale, double* coef, double* part, cudaStream_t st) {
+                  const double2* phase, const double* scale, double* coef, double* part, cudaStream_t st,
+                  const std::function<int(bool)>& stencil) {
     const BrickTables& b = h->pj.bricks;
     if (nk <= 0 || ns <= 0) return QG_OK;
     if (b.nitems == 0) {  // every table value is zero
         QG_CUDA_TRY(cudaMemsetAsync(coef, 0, coef_elems(h, nk, ns, cplx) * sizeof(double), st));
-        return QG_OK;
+        return stencil ? stencil(false) : QG_OK;
     }
     const bool rows = by_rows(b.nitems, slice_units(b, cplx, nk * ((ns + 7) / 8)));
     const bool vec = pairs_ok(h, X, ldx, ldk) && (!cplx || h->N() % 2 == 0);
-#define QG_GO(C, V, R) return launch_project<T, C, V, R>(h, nk, ns, X, ldx, ldk, phase, scale, coef, part, st)
+#define QG_GO(C, V, R) return launch_project<T, C, V, R>(h, nk, ns, X, ldx, ldk, phase, scale, coef, part, st, stencil)
     if (cplx) {
         if (vec && rows) QG_GO(true, true, true);
         if (vec) QG_GO(true, true, false);
@@ -551,12 +562,12 @@ int brick_project(qg_hamiltonian h, int nk, int ns, bool cplx, const T* X, long 
 
 template <typename T>
 int brick_scatter_z(qg_hamiltonian h, int nk, int ns, T* HX, long long ldx, long long ldk, const double2* phase,
-                    const double* coef, cudaStream_t st) {
+                    const double* coef, bool early, cudaStream_t st) {
     const BrickTables& b = h->pj.bricks;
     if (b.nitems == 0 || nk <= 0 || ns <= 0) return QG_OK;
     const bool rows = by_rows(b.nbricks, nk * ((ns + 7) / 8));
     const bool vec = pairs_ok(h, HX, ldx, ldk) && h->N() % 2 == 0;
-#define QG_GO(V, R) return launch_scatter<T, V, R>(h, nk, ns, HX, ldx, ldk, phase, coef, st)
+#define QG_GO(V, R) return launch_scatter<T, V, R>(h, nk, ns, HX, ldx, ldk, phase, coef, early, st)
     if (vec && rows) QG_GO(true, true);
     if (vec) QG_GO(true, false);
     if (rows) QG_GO(false, true);
@@ -565,13 +576,14 @@ int brick_scatter_z(qg_hamiltonian h, int nk, int ns, T* HX, long long ldx, long
 }
 
 template int brick_project<double>(qg_hamiltonian, int, int, bool, const double*, long long, long long, const double2*,
-                                   const double*, double*, double*, cudaStream_t);
+                                   const double*, double*, double*, cudaStream_t,
+                                   const std::function<int(bool)>&);
 template int brick_project<float>(qg_hamiltonian, int, int, bool, const float*, long long, long long, const double2*,
-                                  const double*, double*, double*, cudaStream_t);
+                                  const double*, double*, double*, cudaStream_t, const std::function<int(bool)>&);
 template int brick_scatter_z<double>(qg_hamiltonian, int, int, double*, long long, long long, const double2*,
-                                     const double*, cudaStream_t);
+                                     const double*, bool, cudaStream_t);
 template int brick_scatter_z<float>(qg_hamiltonian, int, int, float*, long long, long long, const double2*,
-                                    const double*, cudaStream_t);
+                                    const double*, bool, cudaStream_t);
 
 int ensure_phases(qg_hamiltonian h, int nk, const double* kv, cudaStream_t st, const double2** out) {
     BrickTables& b = h->pj.bricks;

@@ -1,5 +1,6 @@
 // Nonlocal projectors as FP64 tensor-core contractions over bricks of the grid (nonlocal.cu).
 #pragma once
+#include <functional>
 #include <vector>
 
 #include "qg_internal.h"
@@ -31,14 +32,16 @@ int brick_project_launches(qg_hamiltonian h, int ns);
 
 // Real: coef[(atom * nch + ch) * coef_ld(ns) + s] = scale[atom * nch + ch] * sum_p P(p) psi_s(p).
 // Complex: coef[((k * ncg + cg) * coef_rows + row) * 4 + c], cg = atom * (nch / 4) + channel group;
-// phase: the tables of ensure_phases (real states: nullptr).
+// phase: the tables of ensure_phases (real states: nullptr). stencil (may be empty) launches a kernel that reads
+// X and touches neither coef nor part: beside the projection where it can (early, see launch_kernel).
 template <typename T>
 int brick_project(qg_hamiltonian h, int nk, int ns, bool cplx, const T* X, long long ldx, long long ldk,
-                  const double2* phase, const double* scale, double* coef, double* part, cudaStream_t st);
+                  const double2* phase, const double* scale, double* coef, double* part, cudaStream_t st,
+                  const std::function<int(bool early)>& stencil = {});
 // HX += sum over spheres and channels conj(P) coef, complex states.
 template <typename T>
 int brick_scatter_z(qg_hamiltonian h, int nk, int ns, T* HX, long long ldx, long long ldk, const double2* phase,
-                    const double* coef, cudaStream_t st);
+                    const double* coef, bool early, cudaStream_t st);
 
 // Bloch phases exp(i g.r) of nk k-vectors (HOST, 3 each): per k-point nx + ny + nz values of
 // the axes, then one per periodic image; rebuilt when the k-vectors change.

@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(kConsumers<T> + 32, 1) k_stencil_kpoint(const 
     const int t = threadIdx.x;
     const long long plane = (long long)nx * ny;
 
+    allow_next();
     if (t == 0) {
         for (int i = 0; i < nst; ++i) {
             mbar_init(&full[i], 1);
@@ -280,6 +281,7 @@ __global__ void __launch_bounds__(kConsumers<T> + 32, 1) k_stencil_kpoint(const 
         const int last = ctl[1];
         for (int ps = max(0, last - nst + 1); ps <= last; ++ps) mbar_wait(&full[ps % nst], (uint32_t)(ps / nst) & 1u);
     }
+    wait_previous();
 }
 
 // Ring stages of a tile of ty rows, -1: too few fit (R + 1 planes are held, 2 more in flight).
@@ -342,7 +344,7 @@ int launch_order(const HamArgs<T>& a, cudaStream_t st) {
     wg.zslab = (a.nz + wg.nslab - 1) / wg.nslab;
     wg.nslab = (a.nz + wg.zslab - 1) / wg.zslab;
     wg.items = (int)(base * wg.nslab);
-    kern<<<std::min(G0, wg.items), threads, smem, st>>>(a, wg, nst);
+    QG_CUDA_TRY(launch_kernel(a.early, kern, dim3(std::min(G0, wg.items)), dim3(threads), smem, st, a, wg, nst));
     return QG_OK;
 }
 

@@ -123,6 +123,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_stencil_pair(const HamArgs<
     const int t = threadIdx.x;
     const long long plane = (long long)nx * ny;
 
+    allow_next();
     if (t == 0) {
         for (int i = 0; i < nst; ++i) {
             mbar_init(&full[i], 1);
@@ -297,6 +298,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_stencil_pair(const HamArgs<
         const int last = ctl[1];
         for (int ps = max(0, last - nst + 1); ps <= last; ++ps) mbar_wait(&full[ps % nst], (uint32_t)(ps / nst) & 1u);
     }
+    wait_previous();
 }
 
 // Rows per tile: the largest divisor of ny (<= 16) keeping the consumers within the limit.
@@ -342,7 +344,7 @@ int launch_pair_order(const HamArgs<T>& a, cudaStream_t st) {
     wg.nslab = (a.nz + wg.zslab - 1) / wg.zslab;
     wg.items = (int)(base * wg.nslab);
     const int G = std::min(G0, wg.items);
-    kern<<<G, threads, smem, st>>>(a, wg, nst);
+    QG_CUDA_TRY(launch_kernel(a.early, kern, dim3(G), dim3(threads), smem, st, a, wg, nst));
     return QG_OK;
 }
 
