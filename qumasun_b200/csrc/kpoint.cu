@@ -19,6 +19,16 @@
 namespace qg {
 namespace {
 
+// The per-k-point stencil coefficients of a launch, 32 k-points at a time.
+struct KcoArgs {
+    static constexpr int n = 32 * 13;
+    double v[n];
+};
+template <typename T>
+__global__ void k_store_kco(const KcoArgs args, int n, T* __restrict__ out) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) out[i] = T(args.v[i]);
+}
+
 // Any-shape fallback for V u - 1/2 (Lap + 2i g.grad - g^2) u at FD order 2, 6 or 8: one
 // thread per (point, state), neighbours read from global memory with periodic wrap. The
 // sums follow LaplasianKpoint{2nd,6th,8th}_halo_f (order 2: c0 p + cx (p+x + p-x) + ...;
@@ -173,11 +183,14 @@ int apply_hamiltonian_zk(qg_hamiltonian h, int nk, const double* kv, int nsk, co
         a.dz[d] = T(kc[9 + d]);
     }
     if (nk > 1) {
-        std::vector<T> kct(kc.begin(), kc.end());
-        QG_TRY(h->kco.reserve(kct.size() * sizeof(T)));
-        // the coefficients are read by this launch only; the stream keeps the copy ordered
-        QG_CUDA_TRY(cudaMemcpyAsync(h->kco.ptr, kct.data(), kct.size() * sizeof(T), cudaMemcpyHostToDevice, st));
-        QG_CUDA_TRY(cudaStreamSynchronize(st));  // kct is a host temporary
+        QG_TRY(h->kco.reserve(kc.size() * sizeof(T)));
+        // as kernel arguments: no copy from pageable memory and no synchronisation (12 us of a 62 us call)
+        for (size_t at = 0; at < kc.size(); at += KcoArgs::n) {
+            KcoArgs args;
+            const int n = (int)std::min<size_t>(KcoArgs::n, kc.size() - at);
+            std::copy_n(kc.begin() + at, n, args.v);
+            k_store_kco<T><<<1, 256, 0, st>>>(args, n, h->kco.as<T>() + at);
+        }
         a.kco = h->kco.as<T>();
         a.nsk = nsk;
         a.ldkx = ldk;
