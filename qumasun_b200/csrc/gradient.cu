@@ -13,7 +13,7 @@
 // 139 of 256 states of 80^3 take 0.53 ms (0.35 ms of bytes at the copy rate), against 4.0 ms for
 // 24 neighbour loads per point from L1 (k_gradient8, which stays for the shapes TMA does not take).
 // The same products in the Hamiltonian's stencil measured slower than its vector kernels (1.17
-// against 0.55 ms real, 0.63 against 0.65 k-points): the FP64 tensor and vector instructions share
+// against 0.55 ms real, 0.63 against 0.44 k-points): the FP64 tensor and vector instructions share
 // one pipe, where 16 band products per axis and point cost more than 9 of 13 additions saved.
 //
 // Any ny >= 8 and nx, nz whose rows TMA takes (even nx, 16-byte state strides): a tile past the last
