@@ -141,7 +141,8 @@ __device__ __forceinline__ void load_table(double* tb, const BrickGeom& g, int i
     __syncthreads();
 }
 
-// A unit is 8 states: one group of 8 rows (real) or two, re and im (complex). ROWS: the 8
+// A unit is 8 states, of several k-points where they follow one another (the phase is the lane's): one
+// group of 8 rows (real) or two, re and im (complex). ROWS: the 8
 // warps take one row of the brick each for one unit (few units: more warps per state);
 // otherwise they take one unit each and walk the whole brick, the table in shared memory. Both
 // add a row's blocks first and then the rows in order, so the sums are the same to the bit.
@@ -149,7 +150,7 @@ __device__ __forceinline__ void load_table(double* tb, const BrickGeom& g, int i
 // D blocks of states are in flight per warp.
 template <typename T, bool CPLX, bool VEC, bool ROWS, int D>
 __global__ void __launch_bounds__(kThreads, 2)
-    k_brick_project(const T* __restrict__ X, long long ldx, long long ldk, long long xim, int ns, int per_k,
+    k_brick_project(const T* __restrict__ X, long long ldx, long long ldk, long long xim, int ns, int nrow,
                     int unit0, int nunit, const BrickGeom g, const double2* __restrict__ phase, int nphase,
                     double* __restrict__ part, long long prow) {
     constexpr int S = CPLX ? 2 : 1;
@@ -163,10 +164,10 @@ __global__ void __launch_bounds__(kThreads, 2)
     const int np = g.item_pair[item + 1] - g.item_pair[item];
     const int ul = ROWS ? ch : ch * 8 + w;            // unit of this warp within the launch
     const int u = unit0 + min(ul, nunit - 1);
-    const int k = u / per_k, s = (u - k * per_k) * 8 + r;
+    const int row_r = min(u * 8 + r, nrow - 1), k = row_r / ns, s = row_r - k * ns;  // this lane's state
     const int x = bx * kBx + 2 * q, y0 = by * kBy, z0 = bz * kBz;
     const long long plane = (long long)g.nx * g.ny;
-    const T* base = X + (long long)k * ldk + (long long)min(s, ns - 1) * ldx + (x + (long long)g.nx * y0 + plane * z0);
+    const T* base = X + (long long)k * ldk + (long long)s * ldx + (x + (long long)g.nx * y0 + plane * z0);
     const double2* ph = CPLX ? phase + (long long)k * nphase : nullptr;
 
     using P2 = typename Pair<T>::type;
@@ -273,13 +274,13 @@ __global__ void __launch_bounds__(kThreads, 2)
 template <bool CPLX>
 __global__ void __launch_bounds__(kThreads)
     k_brick_reduce(const double* part, long long prow, const int* __restrict__ cg_off,
-                   const int2* __restrict__ cg_ref, int ncg, int per_k, int unit0, const double2* __restrict__ phase,
+                   const int2* __restrict__ cg_ref, int ns, int nrow, int unit0, const double2* __restrict__ phase,
                    int nphase, int img0, const double* __restrict__ scale, double* __restrict__ coef, long long rows) {
     __shared__ double sm[8][2][32];
     allow_next();
-    const int cg = blockIdx.x, u = unit0 + blockIdx.y, k = u / per_k;
-    const long long lg = u - k * per_k;  // unit of the k-point
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int cg = blockIdx.x, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long u = unit0 + blockIdx.y;
+    const int k = (int)min(u * 8 + (lane >> 2), (long long)nrow - 1) / ns;
     const int r0 = cg_off[cg], n = cg_off[cg + 1] - r0;
     const int b0 = r0 + n * w / 8, b1 = r0 + n * (w + 1) / 8;
     const long long row = (long long)blockIdx.y * (CPLX ? 16 : 8) + (lane >> 2);
@@ -307,8 +308,8 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
         for (int t = 1; t < 8; ++t) v += sm[t][w][lane];
         v *= scale[cg * 4 + (lane & 3)];
-        if constexpr (CPLX) coef[(((long long)k * ncg + cg) * rows + lg * 16 + w * 8) * 4 + lane] = v;
-        else coef[(cg * 4 + (lane & 3)) * rows + lg * 8 + (lane >> 2)] = v;
+        if constexpr (CPLX) coef[(cg * rows + u * 16 + w * 8) * 4 + lane] = v;
+        else coef[(cg * 4 + (lane & 3)) * rows + u * 8 + (lane >> 2)] = v;
     }
 }
 
@@ -316,9 +317,9 @@ __global__ void __launch_bounds__(kThreads)
 // blocks stream by. Units and rows as in k_brick_project.
 template <typename T, bool VEC, bool ROWS, int D>
 __global__ void __launch_bounds__(kThreads, 2)
-    k_brick_scatter(T* __restrict__ HX, long long ldx, long long ldk, long long xim, int ns, int per_k, int nunit,
+    k_brick_scatter(T* __restrict__ HX, long long ldx, long long ldk, long long xim, int ns, int nrow, int nunit,
                     const BrickGeom g, const double2* __restrict__ phase, int nphase, int img0,
-                    const double* coef, int ncg, long long rows) {
+                    const double* coef, long long rows) {
     extern __shared__ __align__(16) double tb[];
     const int chunks = ROWS ? nunit : (nunit + 7) / 8;
     const int brick = blockIdx.x / chunks, ch = blockIdx.x - brick * chunks;
@@ -326,8 +327,8 @@ __global__ void __launch_bounds__(kThreads, 2)
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
     const int ul = ROWS ? ch : ch * 8 + w;
     const int u = min(ul, nunit - 1);
-    const int k = u / per_k, lu = u - k * per_k, s = lu * 8 + r;
-    const bool live = ul < nunit && s < ns;
+    const int row_r = min(u * 8 + r, nrow - 1), k = row_r / ns, s = row_r - k * ns;  // this lane's state
+    const bool live = ul * 8 + r < nrow;
     const int x = bx * kBx + 2 * q, y0 = by * kBy, z0 = bz * kBz;
     const long long plane = (long long)g.nx * g.ny;
     T* base = HX + (long long)k * ldk + (long long)s * ldx + (x + (long long)g.nx * y0 + plane * z0);
@@ -356,7 +357,7 @@ __global__ void __launch_bounds__(kThreads, 2)
             const int cg = g.item_cg[item * 8 + j];
             A[j][0] = A[j][1] = 0.0;
             if (cg >= 0) {
-                const double* c = &coef[(((long long)k * ncg + cg) * rows + lu * 16) * 4 + lane];
+                const double* c = &coef[(cg * rows + u * 16) * 4 + lane];
                 const double re = c[0], im = c[32];
                 const double2 p = __ldg(&ph[img0 + g.item_img[item * 8 + j]]);
                 A[j][0] = p.x * re + p.y * im;
@@ -460,7 +461,7 @@ int launch_project(qg_hamiltonian h, int nk, int ns, const T* X, long long ldx, 
                    const std::function<int(bool)>& stencil) {
     constexpr int D = CPLX ? 4 : 8;
     const BrickTables& b = h->pj.bricks;
-    const int per_k = (ns + 7) / 8, units = nk * per_k, most = slice_units(b, CPLX, units);
+    const int nrow = nk * ns, units = (nrow + 7) / 8, most = slice_units(b, CPLX, units);
     auto kern = k_brick_project<T, CPLX, VEC, ROWS, D>;
     if (allow_max_dynamic_smem(kern) != cudaSuccess) return QG_ERR_CUDA;
     const int np = phase_count(h);
@@ -468,13 +469,13 @@ int launch_project(qg_hamiltonian h, int nk, int ns, const T* X, long long ldx, 
         const int nu = std::min(most, units - u0);
         const long long prow = (long long)nu * (CPLX ? 16 : 8);
         kern<<<(unsigned)((long long)b.nitems * (ROWS ? nu : (nu + 7) / 8)), kThreads, (size_t)b.max_tab * 512, st>>>(
-            X, ldx, ldk, h->N(), ns, per_k, u0, nu, geom(h), phase, np, part, prow);
+            X, ldx, ldk, h->N(), ns, nrow, u0, nu, geom(h), phase, np, part, prow);
         // one slice: the stencil runs beside the projection, and ends after it
         const bool beside = stencil && nu == units;
         if (beside) QG_TRY(stencil(true));
         QG_CUDA_TRY(launch_kernel(beside && small_call((long long)nk * ns * h->N()), k_brick_reduce<CPLX>, dim3(b.ncg, nu),
-                                  dim3(kThreads), 0, st, part, prow, b.cg_off, b.cg_ref, b.ncg, per_k, u0, phase, np,
-                                  h->nx + h->ny + h->nz, scale, coef, coef_rows(ns, CPLX)));
+                                  dim3(kThreads), 0, st, part, prow, b.cg_off, b.cg_ref, ns, nrow, u0, phase, np,
+                                  h->nx + h->ny + h->nz, scale, coef, coef_rows(nrow, CPLX)));
     }
     if (stencil && units > most) QG_TRY(stencil(false));
     QG_CUDA_TRY(cudaGetLastError());
@@ -485,13 +486,13 @@ template <typename T, bool VEC, bool ROWS>
 int launch_scatter(qg_hamiltonian h, int nk, int ns, T* HX, long long ldx, long long ldk, const double2* phase,
                    const double* coef, bool early, cudaStream_t st) {
     const BrickTables& b = h->pj.bricks;
-    const int per_k = (ns + 7) / 8, units = nk * per_k;
+    const int nrow = nk * ns, units = (nrow + 7) / 8;
     auto kern = k_brick_scatter<T, VEC, ROWS, 4>;
     if (allow_max_dynamic_smem(kern) != cudaSuccess) return QG_ERR_CUDA;
     QG_CUDA_TRY(launch_kernel(
         early, kern, dim3((unsigned)((long long)b.nbricks * (ROWS ? units : (units + 7) / 8))), dim3(kThreads),
-        (size_t)b.max_tab * 512, st, HX, ldx, ldk, h->N(), ns, per_k, units, geom(h), phase, phase_count(h), h->nx + h->ny + h->nz, coef, b.ncg,
-        coef_rows(ns, true)));
+        (size_t)b.max_tab * 512, st, HX, ldx, ldk, h->N(), ns, nrow, units, geom(h), phase, phase_count(h), h->nx + h->ny + h->nz, coef,
+        coef_rows(nrow, true)));
     return QG_OK;
 }
 
@@ -509,13 +510,13 @@ int floor_div(int a, int b) { return a >= 0 ? a / b : -((b - 1 - a) / b); }
 }  // namespace
 
 size_t coef_elems(qg_hamiltonian h, int nk, int ns, bool cplx) {
-    return (size_t)nk * h->pj.na * h->pj.nch * coef_rows(ns, cplx);
+    return (size_t)h->pj.na * h->pj.nch * coef_rows(nk * ns, cplx);
 }
 
 size_t part_elems(qg_hamiltonian h, int nk, int ns, bool cplx) {
     const BrickTables& b = h->pj.bricks;
     if (b.nitems == 0 || ns <= 0) return 0;
-    return (size_t)b.npairs * slice_units(b, cplx, nk * ((ns + 7) / 8)) * (cplx ? 16 : 8) * 8;
+    return (size_t)b.npairs * slice_units(b, cplx, (nk * ns + 7) / 8) * (cplx ? 16 : 8) * 8;
 }
 
 // By the cell alone, so that a state's bits never depend on its batch: cells of more than 16 atoms,
@@ -541,7 +542,7 @@ int brick_project(qg_hamiltonian h, int nk, int ns, bool cplx, const T* X, long 
         QG_CUDA_TRY(cudaMemsetAsync(coef, 0, coef_elems(h, nk, ns, cplx) * sizeof(double), st));
         return stencil ? stencil(false) : QG_OK;
     }
-    const bool rows = by_rows(b.nitems, slice_units(b, cplx, nk * ((ns + 7) / 8)));
+    const bool rows = by_rows(b.nitems, slice_units(b, cplx, (nk * ns + 7) / 8));
     const bool vec = pairs_ok(h, X, ldx, ldk) && (!cplx || h->N() % 2 == 0);
 #define QG_GO(C, V, R) return launch_project<T, C, V, R>(h, nk, ns, X, ldx, ldk, phase, scale, coef, part, st, stencil)
     if (cplx) {
@@ -565,7 +566,7 @@ int brick_scatter_z(qg_hamiltonian h, int nk, int ns, T* HX, long long ldx, long
                     const double* coef, bool early, cudaStream_t st) {
     const BrickTables& b = h->pj.bricks;
     if (b.nitems == 0 || nk <= 0 || ns <= 0) return QG_OK;
-    const bool rows = by_rows(b.nbricks, nk * ((ns + 7) / 8));
+    const bool rows = by_rows(b.nbricks, (nk * ns + 7) / 8);
     const bool vec = pairs_ok(h, HX, ldx, ldk) && h->N() % 2 == 0;
 #define QG_GO(V, R) return launch_scatter<T, V, R>(h, nk, ns, HX, ldx, ldk, phase, coef, early, st)
     if (vec && rows) QG_GO(true, true);

@@ -14,7 +14,7 @@ int build_bricks(qg_hamiltonian h, const std::vector<int>& atom_off, const std::
                  const std::vector<std::vector<double>>& tabs);
 void free_bricks(BrickTables& b);
 
-// Rows of projector coefficients per k-point: the state count rounded up to 16 (real), or
+// Rows of projector coefficients: the count of states (of all k-points) rounded up to 16 (real), or
 // {re, im} in alternating groups of 8 (complex).
 inline long long coef_rows(int ns, bool cplx) { return cplx ? 16LL * ((ns + 7) / 8) : coef_ld(ns); }
 
@@ -31,7 +31,7 @@ inline size_t nonlocal_scratch(qg_hamiltonian h, int nk, int ns, bool cplx) {
 int brick_project_launches(qg_hamiltonian h, int ns);
 
 // Real: coef[(atom * nch + ch) * coef_ld(ns) + s] = scale[atom * nch + ch] * sum_p P(p) psi_s(p).
-// Complex: coef[((k * ncg + cg) * coef_rows + row) * 4 + c], cg = atom * (nch / 4) + channel group;
+// Complex: coef[(cg * coef_rows + row) * 4 + c], cg = atom * (nch / 4) + channel group;
 // phase: the tables of ensure_phases (real states: nullptr). stencil (may be empty) launches a kernel that reads
 // X and touches neither coef nor part: beside the projection where it can (early, see launch_kernel).
 template <typename T>
