@@ -4,7 +4,7 @@
 //
 // A producer lane streams the planes of a work item (state, tile of ty rows, z slab) into a ring of
 // shared-memory stages -- TMA boxes of whole rows (or of 8 ntx + 8 columns, with the 4 wrapped
-// columns of an edge tile in a box of their own): the tile's rows, 4 rows above and 4 below -- and
+// columns of a tile that reaches over an end of the row in a box of their own): the tile's rows, 4 rows above and 4 below -- and
 // the consumer warps release a stage when its last reader has passed. A consumer warp owns 8 x 8
 // points of the plane, lane (r, q) = (lane / 4, lane % 4) the points (y0 + r, x0 + 2 q) and its right
 // neighbour -- the accumulator layout of m8n8k4. Per plane: 16 inputs of 8 outputs in four steps
@@ -49,7 +49,7 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
 }
 
 // Sections of a stage, each on a 128-byte boundary: the 4 rows above the tile, the
-// tile, the 4 rows below, the wrapped columns of an edge tile (elements).
+// tile, the 4 rows below, the wrapped columns (elements).
 struct Sections {
     int pitch, main, below, edge, size;
     __host__ __device__ Sections(int ty, int pitch_, bool split) : pitch(pitch_) {
@@ -133,8 +133,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int y0 = min((tile / a.xsplit) * ty, ny - ty);
             const int xi = tile % a.xsplit, xa = split ? xi * 8 * a.ntx - kHalo : 0;
             const int above = wrap_idx(y0 - kHalo, ny), below = wrap_idx(y0 + ty, ny);
-            // an edge tile's wrapped columns: the last 4 left of the first, the first 4 right of the last
-            const int xe = !split ? -1 : (xi == 0 ? nx - kHalo : (xi == a.xsplit - 1 ? 0 : -1));
+            // wrapped columns: the last 4 left of the first tile, the first 4 right of every tile whose halo ends
+            // past the row (the last one, and the one before a last tile narrower than the halo)
+            const int xe = !split ? -1 : (xi == 0 ? nx - kHalo : ((xi + 1) * 8 * a.ntx + kHalo > nx ? 0 : -1));
             // 4 halo rows that wrap inside come row by row
             const bool ra = above + kHalo > ny, rb = below + kHalo > ny;
             const int xl = max(xa, 0), xn = min(nx, xa + a.pitch) - xl;  // a row's columns inside the grid
@@ -304,6 +305,7 @@ bool plan(GradArgs& a) {
     for (int split = 1; split <= nxt; ++split) {
         const int ntx = (nxt + split - 1) / split;
         if (ntx > maxw || (split > 1 && (nxt + ntx - 1) / ntx != split)) continue;
+        if (split == 2 && 8 * ntx + kHalo > a.nx) continue;  // the first tile would wrap on both sides
         const int cols = split > 1 ? 8 * ntx + 2 * kHalo : a.nx;
         // row pitch in which the 8 rows x 4 inputs of an operand fall into different banks
         int pitch = (cols + 3) / 4 * 4;

@@ -49,3 +49,20 @@ def test_force_matches_oracle(cuda_ctx, name, ns):
     f0, e0, ev0 = H.nonlocal_force(Xd, np.zeros(ns))
     assert np.abs(f0).max() == 0.0 and np.abs(e0 - er).max() < te and ev0 == 0.0
     H.close()
+
+
+@pytest.mark.parametrize("grid", [(130, 56, 8), (130, 100, 8), (146, 40, 9), (128, 40, 8), (144, 24, 10)])
+def test_force_on_rows_cut_into_tiles(cuda_ctx, grid):
+    """Rows the gradient kernel cuts into tiles of 16 or 24 columns: the last tile 2 columns wide (130 and
+    146: the tile before it reads across the row's end too), full ones (128, 144)."""
+    import torch
+    from qumasun_b200 import Hamiltonian
+    cell = build_cell(grid=grid, displacement=0.05, seed=6)
+    X = initial_states(5, cell.N, seed=1)
+    occ = np.array([2.0, 1.5, 0.0, 1.0, 0.25])
+    fr, er, evr = O.nonlocal_force(cell, X, occ, impl="port")
+    H = Hamiltonian(cuda_ctx, cell)
+    f, e, ev = H.nonlocal_force(torch.from_numpy(X).cuda(), occ)
+    H.close()
+    assert np.abs(f - fr).max() < 1e-10 * np.abs(fr).max() and np.abs(e - er).max() < 1e-10 * np.abs(er).max()
+    assert abs(ev - evr) < 1e-10 * abs(evr)
