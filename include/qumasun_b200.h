@@ -411,7 +411,7 @@ int qg_hamiltonian_set_nonlocal_blocking(qg_hamiltonian ham, int project_states,
  * 2n step, rank-revealing solve or rollback; 0 forms the full Gram every iteration. */
 int qg_hamiltonian_set_gram_reuse(qg_hamiltonian ham, int on);
 /* Test hook of the bounded waits: with on = 1 the producer lane of the ring stencil
- * kernels (real states) issues no copy, so every consumer's bounded mbarrier wait
+ * kernels (real states) and of the forces' gradient kernel issues no copy, so every consumer's bounded mbarrier wait
  * (about 2^31 SM clocks) runs out; the kernels then wind down, record QG_ERR_TIMEOUT
  * in the context's device status word (qg_context_synchronize /
  * qg_context_take_device_status) and the context stays usable. 0 restores normal
@@ -493,7 +493,9 @@ int qg_td_taylor4_z(qg_hamiltonian ham, int ns, double dt, double* X, long long 
  * occ[s] > 0, dpsi = -2 occ grad psi (8th-order FD gradient, Gradient8th,
  * GridGradient8th.h:19-235), dinner = dV <p|dpsi> and forces[3a + d] +=
  * sum E inner dinner_d; *ev_sum = sum occ[s] e_state[s]. occ, forces (3 per atom,
- * accumulated), e_state (may be NULL) and ev_sum (may be NULL) are HOST. Replaces
+ * accumulated), e_state (may be NULL) and ev_sum (may be NULL) are HOST. QG_ERR_TIMEOUT (a
+ * bounded wait on the device ran out, here or in an earlier launch) leaves forces and e_state
+ * as they were. Replaces
  * QUMASUN_MPI::mGetForcePseudoNonlocal (qumasun_mpi.force.h:227-254) with
  * PseudoPotIntegrator_mpi::ForceNonlocal (PseudoPotOperator_mpi_v2.h:905-1010). */
 int qg_nonlocal_force_d(qg_hamiltonian ham, int ns, const double* X, long long ldx, const double* occ,

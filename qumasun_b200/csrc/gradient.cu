@@ -81,6 +81,7 @@ struct GradArgs {
     int xsplit;       // tiles along x; 1: whole rows, stored from x = 0
     int nst;          // ring stages
     int* err;
+    int stall;        // test hook: the producer issues nothing
 };
 
 __device__ __forceinline__ void tma_box(void* dst, const CUtensorMap* map, int x, int y, int z, int s, uint64_t* bar) {
@@ -124,7 +125,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (t < 32) {
         // ---------------- producer ----------------
         int pos = 0;
-        for (int item = blockIdx.x; item < wg.items && t == 0; item += gridDim.x) {
+        for (int item = blockIdx.x; item < wg.items && t == 0 && !a.stall; item += gridDim.x) {
             const int slab = item % wg.nslab;
             const int tile = (item / wg.nslab) % wg.tiles;
             const int s = a.sidx[item / (wg.nslab * wg.tiles)];
@@ -332,8 +333,8 @@ bool plan(GradArgs& a) {
 }  // namespace
 
 int launch_gradient8(const double* X, long long ldx, int nin, const int* sidx, int ns, double* out, int nx, int ny, int nz,
-                     const double* h, int* err, cudaStream_t st) {
-    GradArgs a{X, ldx, sidx, out, ns, nx, ny, nz, 0, {}, 0, 0, 0, 0, err};
+                     const double* h, int* err, int stall, cudaStream_t st) {
+    GradArgs a{X, ldx, sidx, out, ns, nx, ny, nz, 0, {}, 0, 0, 0, 0, err, stall};
     for (int d = 0; d < 3; ++d) a.s[d] = 672.0 / (840.0 * h[d]);
     tchost::EncodeTiledFn enc = tchost::encode_fn();
     if (!enc || nx % 2 || ldx % 2 || (uintptr_t)X % 16 || (uintptr_t)out % 16 || !plan(a)) return QG_ERR_UNSUPPORTED;

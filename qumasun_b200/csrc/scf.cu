@@ -15,6 +15,7 @@
 #include <cufft.h>
 
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "nonlocal.h"
@@ -516,14 +517,15 @@ int qg_nonlocal_force_d(qg_hamiltonian h, int ns, const double* X, long long ldx
     const size_t ce = qg::coef_elems(h, 1, ns, false), de = qg::coef_elems(h, 1, 3 * nc_max, false);
     const size_t pe = std::max(qg::part_elems(h, 1, ns, false), qg::part_elems(h, 1, 3 * nc_max, false));
     const size_t grad_elems = nu > 0 ? ((size_t)3 * nc_max * N + 1) / 2 * 2 : 0;  // what follows stays 16-byte aligned
-    QG_TRY(h->scf_work.reserve((grad_elems + ce + de + pe + 3 * (size_t)na + ns + 2 * (size_t)nu) * sizeof(double)));
+    QG_TRY(h->scf_work.reserve((grad_elems + ce + de + pe + 3 * (size_t)na + ns + 1 + 2 * (size_t)nu) * sizeof(double)));
     double* grad = h->scf_work.as<double>();
     double* inner = grad + grad_elems;
     double* dinner = inner + ce;
     double* part = dinner + de;
-    double* fdev = part + pe;       // forces, then the energies: one copy back
+    double* fdev = part + pe;       // forces, energies and the device status: one copy back
     double* edev = fdev + 3 * (size_t)na;
-    double* odev = edev + ns;
+    double* sdev = edev + ns;
+    double* odev = sdev + 1;
     int* sidx = reinterpret_cast<int*>(odev + nu);
     QG_CUDA_TRY(cudaMemcpyAsync(fdev, forces, 3 * (size_t)na * sizeof(double), cudaMemcpyHostToDevice, st));
     if (nu > 0) {
@@ -536,7 +538,8 @@ int qg_nonlocal_force_d(qg_hamiltonian h, int ns, const double* X, long long ldx
                                                                  edev);
     for (int s0 = 0; s0 < nu; s0 += nc_max) {
         const int nc = std::min(nc_max, nu - s0);
-        const int rc = qg::launch_gradient8(X, ldx, ns, sidx + s0, nc, grad, h->nx, h->ny, h->nz, h3, h->ctx->dev_status, st);
+        const int rc = qg::launch_gradient8(X, ldx, ns, sidx + s0, nc, grad, h->nx, h->ny, h->nz, h3, h->ctx->dev_status,
+                                            h->test_stall, st);
         if (rc == QG_ERR_UNSUPPORTED)  // odd rows: any shape
             qg::k_gradient8<<<qg::grid_for((long long)nc * N), qg::kThreads, 0, st>>>(
                 h->nx, h->ny, h->nz, nc, X, ldx, sidx + s0, 1.0 / (840.0 * h3[0]), 1.0 / (840.0 * h3[1]),
@@ -547,9 +550,13 @@ int qg_nonlocal_force_d(qg_hamiltonian h, int ns, const double* X, long long ldx
                                                         qg::coef_rows(3 * nc, false), dinner, h->pj.ch_E, fdev);
     }
     QG_CUDA_TRY(cudaGetLastError());
-    std::vector<double> back(3 * (size_t)na + ns);
+    QG_CUDA_TRY(cudaMemcpyAsync(sdev, h->ctx->dev_status, sizeof(int), cudaMemcpyDeviceToDevice, st));
+    std::vector<double> back(3 * (size_t)na + ns + 1);
     QG_CUDA_TRY(cudaMemcpyAsync(back.data(), fdev, back.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     QG_CUDA_TRY(cudaStreamSynchronize(st));
+    int status;
+    std::memcpy(&status, &back.back(), sizeof(int));
+    if (status != 0) return qg_context_take_device_status(h->ctx);  // a wait of the gradient kernel ran out
     std::copy_n(back.data(), 3 * (size_t)na, forces);
     const double* e = back.data() + 3 * (size_t)na;
     if (e_state) std::copy_n(e, ns, e_state);

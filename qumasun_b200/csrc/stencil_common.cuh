@@ -108,8 +108,8 @@ bool stencil_kpoint_ok(const HamArgs<T>& a, int order);
 
 // 8th-order periodic FD gradient of the listed real states (sidx, DEVICE) of the nin at X (gradient.cu):
 // component d of state s at out + (d * ns + s) * N (Gradient8th, GridGradient8th.h:19-235).
-// QG_ERR_UNSUPPORTED where TMA does not take the rows.
+// QG_ERR_UNSUPPORTED where TMA does not take the rows. err, stall: as in HamArgs.
 int launch_gradient8(const double* X, long long ldx, int nin, const int* sidx, int ns, double* out, int nx, int ny, int nz,
-                     const double* h, int* err, cudaStream_t st);
+                     const double* h, int* err, int stall, cudaStream_t st);
 
 }  // namespace qg

@@ -66,3 +66,33 @@ def test_force_on_rows_cut_into_tiles(cuda_ctx, grid):
     H.close()
     assert np.abs(f - fr).max() < 1e-10 * np.abs(fr).max() and np.abs(e - er).max() < 1e-10 * np.abs(er).max()
     assert abs(ev - evr) < 1e-10 * abs(evr)
+
+
+def test_force_reports_a_wait_that_ran_out(cuda_ctx):
+    """With the test hook on, the gradient kernel's producer issues nothing and its consumers give up after
+    about a second: the call returns QG_ERR_TIMEOUT and leaves forces and energies alone."""
+    import torch
+    from qumasun_b200 import Hamiltonian
+    from qumasun_b200.engine import lib
+    cell = build_cell(grid=(16, 16, 16))
+    X = initial_states(3, cell.N, seed=2)
+    occ = np.array([2.0, 1.0, 0.5])
+    H = Hamiltonian(cuda_ctx, cell)
+    Xd = torch.from_numpy(X).cuda()
+    good = H.nonlocal_force(Xd, occ)
+    f, e, ev = np.full(3 * cell.n_atoms, 7.0), np.full(3, 8.0), C.c_double()
+    dp = C.POINTER(C.c_double)
+
+    def call():
+        return lib().qg_nonlocal_force_d(H.h, 3, C.c_void_p(Xd.data_ptr()), cell.N, occ.ctypes.data_as(dp),
+                                         f.ctypes.data_as(dp), e.ctypes.data_as(dp), C.byref(ev))
+
+    assert lib().qg_hamiltonian_test_stall(H.h, 1) == 0
+    assert call() == -5  # QG_ERR_TIMEOUT
+    assert (f == 7.0).all() and (e == 8.0).all()
+    assert lib().qg_hamiltonian_test_stall(H.h, 0) == 0
+    assert call() == 0
+    assert np.abs(f - 7.0 - good[0].reshape(-1)).max() < 1e-14 * 8.0 + 1e-13 * np.abs(good[0]).max()
+    assert np.array_equal(e, good[1]) and ev.value == good[2]
+    assert cuda_ctx.take_device_status() == 0
+    H.close()
