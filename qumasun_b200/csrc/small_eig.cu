@@ -516,13 +516,19 @@ __device__ bool heg_jacobi(int k, SmemHeg& m) {
                     if (q < k) {
                         const double2 cpq = C[p * k + q];
                         const double a2 = cpq.x * cpq.x + cpq.y * cpq.y;
-                        if (a2 != 0.0) {
+                        if (cpq.x != 0.0 || cpq.y != 0.0) {
                             // t = sgn(d) h / (|d| + sqrt(d^2 + h^2)), d = C_qq - C_pp, h = 2 |C_pq|
                             const double d = C[q * k + q].x - C[p * k + p].x;
-                            const double root = sqrt(d * d + 4.0 * a2), apq = sqrt(a2);
-                            const double tt = (d >= 0.0 ? 2.0 : -2.0) * apq / (fabs(d) + root);
-                            const double inv = 1.0 / apq;
+                            double apq = sqrt(a2), root = sqrt(d * d + 4.0 * a2), inv = 1.0 / apq;
                             ph = make_double2(cpq.x * inv, -cpq.y * inv);
+                            if (a2 < 1e-290) {  // |C_pq| < 1e-145: its square loses bits or vanishes
+                                const double x = cpq.x * 0x1p600, y = cpq.y * 0x1p600;
+                                inv = 1.0 / sqrt(x * x + y * y);
+                                ph = make_double2(x * inv, -y * inv);
+                                apq = sqrt(x * x + y * y) * 0x1p-600;
+                                root = hypot(d, 2.0 * apq);
+                            }
+                            const double tt = (d >= 0.0 ? 2.0 : -2.0) * apq / (fabs(d) + root);
                             cs.x = 1.0 / sqrt(1.0 + tt * tt);
                             cs.y = tt * cs.x;
                         }
