@@ -465,9 +465,11 @@ __global__ void __launch_bounds__(256, SG <= 4 ? 3 : 2) k_scatter_all(T* __restr
     constexpr int VN = Vec16<T>::n;
     static_assert(SG % VN == 0, "state group must be whole vectors");
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= N) return;
-    const int e0 = row[g], ne = row[g + 1] - e0;
-    if (ne == 0) return;
+    const int e0 = g < N ? row[g] : 0, ne = g < N ? row[g + 1] - e0 : 0;
+    if (ne == 0) {
+        wait_previous();  // where no point has an entry the grid still ends after the stencil
+        return;
+    }
     int cb[KMAX];  // first coefficient row of the entry's atom
     T v[KMAX][NCH];
 #pragma unroll
@@ -558,9 +560,11 @@ __global__ void __launch_bounds__(256, 2) k_scatter_pairs(T* __restrict__ HX, lo
     using P = typename Pair2<T>::type;
     constexpr int VN = Vec16<T>::n;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npairs) return;
-    const int e0 = row[i], ne = row[i + 1] - e0;
-    if (ne == 0) return;
+    const int e0 = i < npairs ? row[i] : 0, ne = i < npairs ? row[i + 1] - e0 : 0;
+    if (ne == 0) {
+        wait_previous();  // as in k_scatter_all
+        return;
+    }
     const P* ev = reinterpret_cast<const P*>(ent_val);
     int cb[KMAX];  // first coefficient row of the entry's atom
     P v[KMAX][NCH];

@@ -146,3 +146,25 @@ def test_odd_grid_split_scatter_matches_oracle(cuda_ctx, kw, f64):
     got = H.apply(torch.from_numpy(X).cuda().to(torch.float64 if f64 else torch.float32)).double().cpu().numpy()
     H.close()
     assert rel(got, O.hamiltonian_apply(cell, X)) < (1e-12 if f64 else 2e-6)
+
+
+@pytest.mark.parametrize("f64", [True, False], ids=["f64", "f32"])
+@pytest.mark.parametrize("kw", [dict(grid=(16, 12, 10)), dict(reps=(1, 1, 3), grid=(16, 16, 48)), dict(grid=(54, 54, 104))],
+                         ids=["atoms", "bricks", "pairs"])
+def test_projectors_without_a_point(cuda_ctx, kw, f64):
+    """All projector values zero: no grid point has an entry, the scatter launched beside the stencil has
+    nothing to add, and what follows on the stream still follows the stencil."""
+    import torch
+    from qumasun_b200 import Hamiltonian
+    cell = build_cell(**kw)
+    cell.cubes = [[(b, s, 0.0 * w) for b, s, w in at] for at in cell.cubes]
+    bare = build_cell(**kw, nonlocal_on=False)
+    X = torch.from_numpy(initial_states(6, cell.N, seed=8)).cuda().to(torch.float64 if f64 else torch.float32)
+    H, H0 = Hamiltonian(cuda_ctx, cell), Hamiltonian(cuda_ctx, bare)
+    for _ in range(3):
+        ref = H0.apply(X)
+        out = torch.full_like(X, float("nan"))
+        got = H.apply(X, out).clone()  # the next kernel of the stream reads the result
+        assert torch.equal(got, ref)
+    H.close()
+    H0.close()
