@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(TV) k_conv_fwd(const TI* __restrict__ in, cons
 }
 
 // ---------------- backward pass on the tensor cores (mma.sync m16n8k16, BF16 in, FP32 sums)
-// The FP32 gradients enter as three BF16 pieces (d = d1 + d2 + d3 to 2^-24), the activations and
+// The FP32 gradients enter as three BF16 pieces (d = d1 + d2 + d3 to 2^-24 of d or 5e-41), the activations and
 // weights are BF16 already, so the products are those of the FP32 kernels; the FP32 sums of a
 // tile are added to the running sums with ordinary rounding. Bound: shared-memory reads of the
 // operands (ldmatrix); one layer of 16 x 16 channels at 32 states of 40^3 is 14 G multiply-adds.
@@ -157,8 +157,9 @@ __device__ __forceinline__ void put_pieces(__nv_bfloat16* tile, int piece_elems,
     __align__(16) __nv_bfloat16 p[3][8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        p[0][i] = __float2bfloat16(d[i]);
-        const float r1 = d[i] - __bfloat162float(p[0][i]);
+        // finite values beyond the largest BF16 round towards zero, Inf is one piece (Inf - Inf is NaN)
+        p[0][i] = fabsf(d[i]) > 3.38e38f ? __float2bfloat16_rz(d[i]) : __float2bfloat16(d[i]);
+        const float r1 = isinf(d[i]) ? 0.f : d[i] - __bfloat162float(p[0][i]);
         p[1][i] = __float2bfloat16(r1);
         p[2][i] = __float2bfloat16(r1 - __bfloat162float(p[1][i]));
     }

@@ -34,3 +34,31 @@ def test_gradient_at_tile_edges(cuda_ctx, grid, ns):
         off += n
     assert np.array_equal(nn.gradient(*args)[1], g)  # sums in a fixed order
     nn.close()
+
+
+def test_infinite_layer_gradients_stay_infinite(cuda_ctx):
+    """Loss gradients near the top of FP32 that overflow on their way back through the last layer: with
+    positive weights, activations and inputs every product is +Inf, so every sum is, and none is NaN."""
+    import torch
+    from qumasun_b200 import LearnedPreconditioner
+    rng = np.random.default_rng(11)
+    grid = (8, 8, 4)
+    N = grid[0] * grid[1] * grid[2]
+    layers, first = [], []
+    for ci, co, scale in zip(NN.CIN, NN.COUT, (0.02, 0.005, 0.005, 1e4)):
+        first.append(sum(a.size for a in layers))
+        layers += [scale * rng.uniform(0.5, 1.0, co * ci * 27), 0.01 * rng.uniform(0.5, 1.0, co)]
+    P = np.concatenate(layers).astype(np.float32)
+    R, V = rng.uniform(0.5, 1.0, (1, N)), 4.0 * rng.uniform(0.5, 1.0, N)
+    _, p, rms = NN.forward(P, grid, R, V, 4.0)
+    # t = Y / rms constant, 2 max(p) / (N t^2) = 1e35
+    Y = np.full((1, N), rms[0] * np.sqrt(2.0 * p.max() / (N * 1e35)))
+    nn = LearnedPreconditioner(cuda_ctx)
+    nn.set_params(P)
+    loss, g = nn.gradient(grid, torch.from_numpy(R).cuda(), torch.from_numpy(V).cuda(), 4.0, torch.from_numpy(Y).cuda())
+    nn.close()
+    _, rg = NN.loss_and_grad(P, grid, R, V, 4.0, Y)
+    last = first[3]
+    assert np.linalg.norm(g[last:].astype(float) - rg[last:]) < 2e-2 * np.linalg.norm(rg[last:])
+    assert rg[:last].min() > np.finfo(np.float32).max  # the exact values are beyond FP32
+    assert np.isposinf(g[:last]).all()
