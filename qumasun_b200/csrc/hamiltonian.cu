@@ -465,11 +465,9 @@ __global__ void __launch_bounds__(256, SG <= 4 ? 3 : 2) k_scatter_all(T* __restr
     constexpr int VN = Vec16<T>::n;
     static_assert(SG % VN == 0, "state group must be whole vectors");
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int e0 = g < N ? row[g] : 0, ne = g < N ? row[g + 1] - e0 : 0;
-    if (ne == 0) {
-        wait_previous();  // where no point has an entry the grid still ends after the stencil
-        return;
-    }
+    if (g >= N) return;
+    const int e0 = row[g], ne = row[g + 1] - e0;
+    if (ne == 0) return;
     int cb[KMAX];  // first coefficient row of the entry's atom
     T v[KMAX][NCH];
 #pragma unroll
@@ -560,11 +558,9 @@ __global__ void __launch_bounds__(256, 2) k_scatter_pairs(T* __restrict__ HX, lo
     using P = typename Pair2<T>::type;
     constexpr int VN = Vec16<T>::n;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int e0 = i < npairs ? row[i] : 0, ne = i < npairs ? row[i + 1] - e0 : 0;
-    if (ne == 0) {
-        wait_previous();  // as in k_scatter_all
-        return;
-    }
+    if (i >= npairs) return;
+    const int e0 = row[i], ne = row[i + 1] - e0;
+    if (ne == 0) return;
     const P* ev = reinterpret_cast<const P*>(ent_val);
     int cb[KMAX];  // first coefficient row of the entry's atom
     P v[KMAX][NCH];
@@ -801,7 +797,9 @@ int apply_hamiltonian(qg_hamiltonian h, int ns, const T* X, long long ldx, T* HX
     if (!done) QG_TRY(stencil(together));
     if (nonlocal) {
         if (pt) pt->mark(2, st);
-        QG_TRY(launch_scatter_all<T>(pj, HX, ldhx, ns, N, coef, coef_ld(ns), h->scatter_sg, together && small_call((long long)ns * N), st));
+        // early only where some point has an entry: its threads are the ones that wait for the stencil
+        const bool early = together && pj.nent > 0 && small_call((long long)ns * N);
+        QG_TRY(launch_scatter_all<T>(pj, HX, ldhx, ns, N, coef, coef_ld(ns), h->scatter_sg, early, st));
     }
     if (pt) pt->mark(-1, st);
     QG_CUDA_TRY(cudaGetLastError());
