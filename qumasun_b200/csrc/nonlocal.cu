@@ -410,12 +410,18 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
 }
 
-// Phases of the axes' grid coordinates and of the images for one k-point per blockIdx.y;
-// a = g * h per axis.
-__global__ void k_phase_tables(int nx, int ny, int nz, int nimg, const int* __restrict__ img,
-                               const double* __restrict__ kh, double2* __restrict__ out) {
+// k-vectors of a launch, as kernel arguments: no copy from pageable memory, nothing to wait for, and a stream
+// capture takes the launch.
+struct KVecs {
+    static constexpr int n = 128;
+    double v[3 * n];  // a = g * h per axis
+};
+
+// Phases of the axes' grid coordinates and of the images for one k-point per blockIdx.y.
+__global__ void k_phase_tables(int nx, int ny, int nz, int nimg, const int* __restrict__ img, const KVecs kh,
+                               double2* __restrict__ out) {
     const int n = nx + ny + nz + nimg;
-    const double ax = kh[3 * blockIdx.y], ay = kh[3 * blockIdx.y + 1], az = kh[3 * blockIdx.y + 2];
+    const double ax = kh.v[3 * blockIdx.y], ay = kh.v[3 * blockIdx.y + 1], az = kh.v[3 * blockIdx.y + 2];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double th;
         if (i < nx) th = ax * i;
@@ -593,24 +599,22 @@ int ensure_phases(qg_hamiltonian h, int nk, const double* kv, cudaStream_t st, c
     const int n = phase_count(h);
     if (!((int)b.phase_k.size() == 3 * nk && std::equal(kv, kv + 3 * nk, b.phase_k.begin()))) {
         b.phase_k.clear();
-        const size_t head = ((size_t)3 * nk * sizeof(double) + 15) / 16 * 16;
-        QG_TRY(b.phase.reserve(head + (size_t)nk * n * sizeof(double2)));
-        std::vector<double> kh((size_t)3 * nk);
-        for (int k = 0; k < nk; ++k) {
-            kh[3 * k] = kv[3 * k] * h->hx;
-            kh[3 * k + 1] = kv[3 * k + 1] * h->hy;
-            kh[3 * k + 2] = kv[3 * k + 2] * h->hz;
+        QG_TRY(b.phase.reserve((size_t)nk * n * sizeof(double2)));
+        for (int k0 = 0; k0 < nk; k0 += KVecs::n) {
+            const int m = std::min(KVecs::n, nk - k0);
+            KVecs kh;
+            for (int k = 0; k < m; ++k) {
+                kh.v[3 * k] = kv[3 * (k0 + k)] * h->hx;
+                kh.v[3 * k + 1] = kv[3 * (k0 + k) + 1] * h->hy;
+                kh.v[3 * k + 2] = kv[3 * (k0 + k) + 2] * h->hz;
+            }
+            k_phase_tables<<<dim3((n + 127) / 128, m), 128, 0, st>>>(h->nx, h->ny, h->nz, b.nimg, b.img, kh,
+                                                                     b.phase.as<double2>() + (size_t)k0 * n);
         }
-        QG_CUDA_TRY(cudaMemcpyAsync(b.phase.ptr, kh.data(), kh.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-        QG_CUDA_TRY(cudaStreamSynchronize(st));  // kh is a host temporary
-        b.phase_at = head;
-        k_phase_tables<<<dim3((n + 127) / 128, nk), 128, 0, st>>>(
-            h->nx, h->ny, h->nz, b.nimg, b.img, b.phase.as<double>(),
-            reinterpret_cast<double2*>(b.phase.as<char>() + head));
         QG_CUDA_TRY(cudaGetLastError());
         b.phase_k.assign(kv, kv + 3 * nk);
     }
-    *out = reinterpret_cast<const double2*>(b.phase.as<char>() + b.phase_at);
+    *out = b.phase.as<double2>();
     return QG_OK;
 }
 

@@ -79,7 +79,6 @@ struct BrickTables {
     int2* cg_ref = nullptr;
     int* img = nullptr;      // periodic images, 3 per image
     DevBuf phase;            // Bloch phases of the k-vectors phase_k (ensure_phases)
-    size_t phase_at = 0;
     std::vector<double> phase_k;
 };
 

@@ -77,3 +77,36 @@ def test_taylor_step_with_scalar_updates(cuda_ctx, grid):
     H.close()
     # the oracle's powers of H and these lose a few bits per power: the 1e-12 of the other step test
     assert rel(view.cpu(), torch.from_numpy(x)) < 1e-12
+
+
+@pytest.mark.parametrize("many", [False, True], ids=["one-k", "many-k"])
+def test_new_kvectors_inside_a_graph_capture(cuda_ctx, many):
+    """An application at k-vectors the operator has not seen is made of launches alone, so that a stream
+    capture takes it (the scratch is there after a first call of the same size)."""
+    import torch
+    from qumasun_b200 import Hamiltonian
+    cell = build_cell(grid=(16, 12, 10))
+    nk = 130 if many else 1  # more than one launch holds as arguments
+    kv = np.random.default_rng(2).uniform(-0.3, 0.3, (3, nk, 3))
+    X = torch.from_numpy(initial_states(2 * nk, 2 * cell.N, seed=9).reshape(nk, 2, 2 * cell.N)).cuda()
+    H = Hamiltonian(cuda_ctx, cell)
+
+    def apply(k, out=None):
+        if many:
+            return H.apply_zk(kv[k], X, out)
+        H.set_kvector(kv[k][0])
+        return H.apply_z(X[0], None if out is None else out[0])
+
+    out = torch.empty_like(X)
+    apply(0, out)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        apply(1, out)
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    cuda_ctx.use_torch_stream()
+    apply(2)  # other phases in the operator's table
+    assert torch.equal(out.reshape(apply(1).shape) if many else out[0], apply(1))
+    H.close()
