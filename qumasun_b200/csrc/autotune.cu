@@ -25,7 +25,7 @@ template <typename T>
 int timed_phases(qg_hamiltonian h, int ns, const T* X, long long ldx, T* HX, long long ldhx, int reps,
                  float best[3]) {
     best[0] = best[1] = best[2] = FLT_MAX;
-    QG_TRY(h->coef.reserve(qg::nonlocal_scratch(h, 1, ns, false) * sizeof(double)));
+    QG_TRY(h->coef.reserve(qg::real_scratch<T>(h, ns)));
     void* coef = h->coef.ptr;
     for (int r = 0; r < reps + 1; ++r) {  // the first apply warms caches and the instruction path
         qg::PhaseTimer pt;

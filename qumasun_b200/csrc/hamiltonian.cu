@@ -779,8 +779,7 @@ int apply_hamiltonian(qg_hamiltonian h, int ns, const T* X, long long ldx, T* HX
     const bool together = nonlocal && !pt;  // events between the kernels would order them
     bool done = false;                      // the stencil is launched
     if (nonlocal) {
-        // FP32 states, a forced split of the atoms and the no-allocation entry point go atom by atom
-        bool bricks = !atom_major && h->proj_parts == 0 && bricks_for_real(pj);
+        const bool bricks = !atom_major && real_by_bricks<T>(h);
         if constexpr (sizeof(T) == 8) {
             if (bricks) {
                 QG_TRY(brick_project<T>(h, 1, ns, false, X, ldx, 0, nullptr, pj.ch_scale, coef,
@@ -788,8 +787,6 @@ int apply_hamiltonian(qg_hamiltonian h, int ns, const T* X, long long ldx, T* HX
                                         together ? std::function<int(bool)>(stencil) : std::function<int(bool)>()));
                 done = together;
             }
-        } else {
-            bricks = false;
         }
         if (!bricks) QG_TRY(launch_project<T>(pj, ns, X, ldx, coef, coef_ld(ns), h->proj_sb, h->proj_parts, st));
         if (pt) pt->mark(1, st);
@@ -1067,7 +1064,7 @@ static int apply_device(qg_hamiltonian h, int ns, const T* X, long long ldx, T* 
     if (ldx < N || ldhx < N) return QG_ERR_INVALID;
     if (h->gx != 0.0 || h->gy != 0.0 || h->gz != 0.0) return QG_ERR_INVALID;
     QG_CUDA_TRY(cudaSetDevice(h->ctx->device));
-    QG_TRY(h->coef.reserve(qg::nonlocal_scratch(h, 1, ns, false) * sizeof(double)));
+    QG_TRY(h->coef.reserve(qg::real_scratch<T>(h, ns)));
     return qg::apply_hamiltonian<T>(h, ns, X, ldx, HX, ldhx, h->coef.ptr, h->ctx->stream);
 }
 
@@ -1152,7 +1149,7 @@ int qg_hamiltonian_apply_timed_d(qg_hamiltonian h, int ns, const double* X, long
     const long long N = h->N();
     if (ldx < N || ldhx < N) return QG_ERR_INVALID;
     QG_CUDA_TRY(cudaSetDevice(h->ctx->device));
-    QG_TRY(h->coef.reserve(qg::nonlocal_scratch(h, 1, ns, false) * sizeof(double)));
+    QG_TRY(h->coef.reserve(qg::real_scratch<double>(h, ns)));
     qg::PhaseTimer pt;
     const int rc = qg::apply_hamiltonian<double>(h, ns, X, ldx, HX, ldhx, h->coef.ptr, h->ctx->stream, &pt);
     if (rc != QG_OK) return rc;
@@ -1193,7 +1190,7 @@ int qg_hamiltonian_launches_per_apply(qg_hamiltonian h, int ns) {
     const bool nonlocal = h->pj.na > 0 && h->pj.nch > 0;
     if (!nonlocal) return 1;
     // projection, stencil + V, nonlocal scatter
-    return (h->proj_parts == 0 && qg::bricks_for_real(h->pj) ? qg::brick_project_launches(h, ns) : 1) + 2;
+    return (qg::real_by_bricks<double>(h) ? qg::brick_project_launches(h, ns) : 1) + 2;
 }
 
 int qg_hamiltonian_apply_host_d(qg_hamiltonian h, int ns, const double* X, double* HX) {

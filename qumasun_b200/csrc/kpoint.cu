@@ -259,7 +259,7 @@ int apply_z_checked(qg_hamiltonian h, int ns, const T* X, long long ldx, T* HX, 
     if (ldx < 2 * N || ldhx < 2 * N) return QG_ERR_INVALID;
     if (h->order != 2 && h->order != 6 && h->order != 8) return QG_ERR_UNSUPPORTED;
     QG_CUDA_TRY(cudaSetDevice(h->ctx->device));
-    QG_TRY(h->coef.reserve(qg::nonlocal_scratch(h, 1, ns, true) * sizeof(double)));
+    QG_TRY(h->coef.reserve(qg::kpoint_scratch(h, 1, ns)));
     double* coef = h->coef.as<double>();
     return qg::apply_hamiltonian_z<T>(h, ns, X, ldx, HX, ldhx, coef, h->ctx->stream);
 }
@@ -274,7 +274,7 @@ int apply_zk_checked(qg_hamiltonian h, int nk, const double* kvecs, int nsk, con
     if (nk > 1 && (ldk < (long long)nsk * ldx || ldkh < (long long)nsk * ldhx)) return QG_ERR_INVALID;
     if (h->order != 2 && h->order != 6 && h->order != 8) return QG_ERR_UNSUPPORTED;
     QG_CUDA_TRY(cudaSetDevice(h->ctx->device));
-    QG_TRY(h->coef.reserve(qg::nonlocal_scratch(h, nk, nsk, true) * sizeof(double)));
+    QG_TRY(h->coef.reserve(qg::kpoint_scratch(h, nk, nsk)));
     double* coef = h->coef.as<double>();
     return qg::apply_hamiltonian_zk<T>(h, nk, kvecs, nsk, X, ldx, ldk, HX, ldhx, ldkh, coef, h->ctx->stream);
 }
@@ -308,7 +308,7 @@ int qg_hamiltonian_apply_timed_z(qg_hamiltonian h, int ns, const double* X, long
     if (ldx < 2 * N || ldhx < 2 * N) return QG_ERR_INVALID;
     if (h->order != 2 && h->order != 6 && h->order != 8) return QG_ERR_UNSUPPORTED;
     QG_CUDA_TRY(cudaSetDevice(h->ctx->device));
-    QG_TRY(h->coef.reserve(qg::nonlocal_scratch(h, 1, ns, true) * sizeof(double)));
+    QG_TRY(h->coef.reserve(qg::kpoint_scratch(h, 1, ns)));
     double* coef = h->coef.as<double>();
     qg::PhaseTimer pt;
     QG_TRY(qg::apply_hamiltonian_z(h, ns, X, ldx, HX, ldhx, coef, h->ctx->stream, &pt));

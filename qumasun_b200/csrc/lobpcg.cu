@@ -459,7 +459,7 @@ struct Solver {
             lwork = std::max(lwork, lw2);
             QG_TRY(work.reserve((size_t)std::max(lwork, 1) * sizeof(cuDoubleComplex)));
         }
-        QG_TRY(h->coef.reserve(qg::nonlocal_scratch(h, 1, n, c == 2) * sizeof(double)));
+        QG_TRY(h->coef.reserve(c == 1 ? qg::real_scratch<double>(h, n) : qg::kpoint_scratch(h, 1, n)));
         if (mixed) QG_TRY(mg.setup(N, (int)g3, mixed_pieces));
         if (i8 && c == 1) QG_TRY(mg.setup(N, (int)g3, qg::kI8Slices));
         if (c == 1) {
@@ -1149,7 +1149,7 @@ int run_lobpcg_zk(qg_hamiltonian h, const qg_lobpcg_options* opt, int nk, const 
         s.lwork = std::max(lw1, lw2);
         QG_TRY(s.work.reserve((size_t)std::max(s.lwork, 1) * sizeof(cuDoubleComplex)));
     }
-    QG_TRY(h->coef.reserve(qg::nonlocal_scratch(h, nk, nb, true) * sizeof(double)));
+    QG_TRY(h->coef.reserve(qg::kpoint_scratch(h, nk, nb)));
     if (2 * nb <= qg::kGramTsMax) QG_TRY(s.gts.reserve(qg::gram_ts_scratch_doubles(N, nk, true) * sizeof(double)));
     // pencils of up to kSmallHegMax rows: all k-points' Hermitian pencils in one launch
     // of the one-block Jacobi solver (small_eig.cu), cuSOLVER's zhegvd per k-point

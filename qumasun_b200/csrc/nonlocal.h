@@ -24,8 +24,20 @@ size_t coef_elems(qg_hamiltonian h, int nk, int ns, bool cplx);
 size_t part_elems(qg_hamiltonian h, int nk, int ns, bool cplx);
 // Whether real FP64 states are projected brick by brick (see the rule at its definition).
 bool bricks_for_real(const DevProjectors& pj);
-inline size_t nonlocal_scratch(qg_hamiltonian h, int nk, int ns, bool cplx) {
-    return coef_elems(h, nk, ns, cplx) + (cplx || bricks_for_real(h->pj) ? part_elems(h, nk, ns, cplx) : 0);
+// The same for real states of type T under the operator's blocking: FP32 states and a forced split of the atoms
+// go atom by atom, straight into the coefficients.
+template <typename T>
+bool real_by_bricks(qg_hamiltonian h) {
+    return sizeof(T) == sizeof(double) && h->proj_parts == 0 && bricks_for_real(h->pj);
+}
+// Bytes of scratch of an application to real states of type T, and to nk x ns k-point states.
+template <typename T>
+size_t real_scratch(qg_hamiltonian h, int ns) {
+    return real_by_bricks<T>(h) ? (coef_elems(h, 1, ns, false) + part_elems(h, 1, ns, false)) * sizeof(double)
+                                : coef_scratch_elems(h, ns) * sizeof(T);
+}
+inline size_t kpoint_scratch(qg_hamiltonian h, int nk, int ns) {
+    return (coef_elems(h, nk, ns, true) + part_elems(h, nk, ns, true)) * sizeof(double);
 }
 // Kernels brick_project launches for ns real states.
 int brick_project_launches(qg_hamiltonian h, int ns);

@@ -247,20 +247,20 @@ inline long long coef_ld(int ns) { return (ns + 15) / 16 * 16; }
 // Elements of projector-coefficient scratch ([n_atoms * n_channels][coef_ld(ns)]) one apply of ns states needs.
 size_t coef_scratch_elems(qg_hamiltonian h, int ns);
 
-// scratch: nonlocal_scratch(h, 1, ns, false) doubles (nonlocal.h), or coef_scratch_elems(h, ns) of
+// scratch: real_scratch<T>(h, ns) bytes (nonlocal.h), or coef_scratch_elems(h, ns) of
 // T with atom_major, which projects atom by atom straight into the coefficients.
 template <typename T>
 int apply_hamiltonian(qg_hamiltonian h, int ns, const T* X, long long ldx, T* HX, long long ldhx,
                       void* scratch, cudaStream_t st, PhaseTimer* pt = nullptr, bool atom_major = false);
 
 // Complex k-point H (kpoint.cu): state s has its real part at X + s*ldx and its
-// imaginary part N elements later; scratch holds nonlocal_scratch(h, 1, ns, true) doubles.
+// imaginary part N elements later; scratch holds kpoint_scratch(h, 1, ns) bytes.
 template <typename T>
 int apply_hamiltonian_z(qg_hamiltonian h, int ns, const T* X, long long ldx, T* HX, long long ldhx,
                         double* scratch, cudaStream_t st, PhaseTimer* pt = nullptr);
 // Several k-points in one pass: nk k-vectors kv (3 each, bohr^-1), nsk states per k-point,
 // state s of k-point k at X + k*ldk + s*ldx (HX + k*ldkh + s*ldhx); scratch holds
-// nonlocal_scratch(h, nk, nsk, true) doubles.
+// kpoint_scratch(h, nk, nsk) bytes.
 template <typename T>
 int apply_hamiltonian_zk(qg_hamiltonian h, int nk, const double* kv, int nsk, const T* X, long long ldx,
                          long long ldk, T* HX, long long ldhx, long long ldkh, double* scratch, cudaStream_t st,

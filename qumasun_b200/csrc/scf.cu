@@ -472,7 +472,7 @@ int qg_td_taylor4_z(qg_hamiltonian h, int ns, double dt, double* X, long long ld
     QG_TRY(h->scf_work.reserve((size_t)2 * ns * ldw * sizeof(double)));
     double* W1 = h->scf_work.as<double>();
     double* W2 = W1 + (size_t)ns * ldw;
-    QG_TRY(h->coef.reserve(qg::nonlocal_scratch(h, 1, ns, true) * sizeof(double)));
+    QG_TRY(h->coef.reserve(qg::kpoint_scratch(h, 1, ns)));
     double* coef = h->coef.as<double>();
     const double c2 = dt * dt / 2.0;
     const double c3 = c2 * dt / 3.0;

@@ -168,3 +168,28 @@ def test_projectors_without_a_point(cuda_ctx, kw, f64):
         assert torch.equal(got, ref)
     H.close()
     H0.close()
+
+
+def used_by(f):
+    """Device memory that f takes (kept alive by its result)."""
+    import torch
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    keep = f()
+    torch.cuda.synchronize()
+    return before - torch.cuda.mem_get_info()[0], keep
+
+
+def test_single_precision_apply_takes_no_brick_scratch(cuda_ctx):
+    """FP32 states are projected atom by atom: the scratch is their coefficients, FP32, and no partial sums."""
+    import torch
+    from qumasun_b200 import Hamiltonian
+    cell = build_cell(reps=(2, 2, 2), grid=(48, 48, 48))
+    ns = 512
+    H = Hamiltonian(cuda_ctx, cell)
+    H.apply(torch.zeros(16, cell.N, dtype=torch.float32, device="cuda"))
+    X = torch.zeros(ns, cell.N, dtype=torch.float32, device="cuda")
+    out = torch.empty_like(X)
+    taken, _ = used_by(lambda: H.apply_device(ns, X.data_ptr(), out.data_ptr(), cell.N, cell.N, "f32"))
+    assert taken <= 4 * ns * cell.n_atoms * 4 + (4 << 20)
+    H.close()
