@@ -619,18 +619,19 @@ __global__ void __launch_bounds__(256, 2) k_scatter_pairs(T* __restrict__ HX, lo
     }
 }
 
-// Pairs where the rows can be read two points at a time and the pairs are many enough to fill the SMs
-// (one wave of two blocks per SM).
+// Grids with enough pairs of points to fill the SMs (one wave of two blocks per SM); others have no pair tables.
+static bool enough_pairs(long long N) { return N % 2 == 0 && N / 2 >= 2LL * 148 * 256; }
+
+// Pairs where the tables are there and the rows can be read two points at a time.
 template <typename T>
-static bool scatter_by_pairs(const DevProjectors& pj, const T* HX, long long ldhx, long long N) {
-    return pj.pair_row && N % 2 == 0 && ldhx % 2 == 0 && (uintptr_t)HX % (2 * sizeof(T)) == 0 &&
-           N / 2 >= 2LL * 148 * 256;
+static bool scatter_by_pairs(const DevProjectors& pj, const T* HX, long long ldhx) {
+    return pj.pair_row && ldhx % 2 == 0 && (uintptr_t)HX % (2 * sizeof(T)) == 0;
 }
 
 template <typename T>
 static int launch_scatter_all(const DevProjectors& pj, T* HX, long long ldhx, int ns, long long N, const T* coef,
                               long long ldc, int forced_sg, bool early, cudaStream_t st) {
-    if (scatter_by_pairs<T>(pj, HX, ldhx, N)) {
+    if (scatter_by_pairs<T>(pj, HX, ldhx)) {
         const T* ev;
         if constexpr (sizeof(T) == 8) ev = reinterpret_cast<const T*>(pj.pair_val_d);
         else ev = reinterpret_cast<const T*>(pj.pair_val_f);
@@ -938,7 +939,7 @@ int build_projectors(qg_hamiltonian h, const qg_hamiltonian_desc* d) {
     // images has an entry for each): pair_val[e * nch + ch] = {value at 2 i, value at 2 i + 1}
     std::vector<int> pair_row, pair_atom;
     std::vector<double> pair_val;
-    if (nch == 4 && N % 2 == 0) {
+    if (nch == 4 && qg::enough_pairs(N)) {
         pair_row.reserve(N / 2 + 1);
         pair_row.push_back(0);
         for (long long i = 0; i < N / 2; ++i) {

@@ -103,7 +103,7 @@ struct DevProjectors {
     int* ent_atom = nullptr;
     double* ent_val_d = nullptr;
     float* ent_val_f = nullptr;
-    int* pair_row = nullptr;       // the same entries per pair of points (4 channels, even N; else null)
+    int* pair_row = nullptr;       // the same entries per pair of points (4 channels, many points; else null)
     int* pair_atom = nullptr;
     double* pair_val_d = nullptr;
     float* pair_val_f = nullptr;

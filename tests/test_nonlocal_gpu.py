@@ -193,3 +193,17 @@ def test_single_precision_apply_takes_no_brick_scratch(cuda_ctx):
     taken, _ = used_by(lambda: H.apply_device(ns, X.data_ptr(), out.data_ptr(), cell.N, cell.N, "f32"))
     assert taken <= 4 * ns * cell.n_atoms * 4 + (4 << 20)
     H.close()
+
+
+def test_small_grids_hold_no_tables_of_point_pairs(cuda_ctx):
+    """Grids below the size of the two-points scatter: the tables that it alone reads are not built."""
+    from qumasun_b200 import Hamiltonian
+    cell = build_cell(reps=(2, 2, 2), grid=(52, 52, 54))  # 146,016 points
+    taken, H = used_by(lambda: Hamiltonian(cuda_ctx, cell))
+    H.close()
+    assert cell.N < 2 * 2 * 148 * 256  # two points per thread, two blocks of 256 per SM
+    # sphere points: nonzero in any channel of an atom
+    points = sum(int((cell.cubes[a][0][2].reshape(-1) != 0.0).sum()) for a in range(cell.n_atoms))
+    # per sphere point: two orders of 4 channels in FP64 and FP32 and their indices; the bricks' blocks,
+    # up to twice as many FP64 values; the potential and per-point rows
+    assert taken <= points * (2 * 4 * 12 + 2 * 4 + 2 * 4 * 8) + cell.N * 20 + (12 << 20)
