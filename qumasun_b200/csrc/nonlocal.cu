@@ -40,7 +40,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <unordered_map>
 
 #include "stencil_common.cuh"
 
@@ -626,66 +625,59 @@ void free_bricks(BrickTables& b) {
     b = BrickTables();
 }
 
-int build_bricks(qg_hamiltonian h, const std::vector<int>& atom_off, const std::vector<int>& u,
-                 const std::vector<std::vector<double>>& tabs) {
-    BrickTables& b = h->pj.bricks;
+BrickLists list_bricks(const int (&n)[3], const std::vector<int>& atom_off, const std::vector<int>& u,
+                       const std::vector<std::vector<double>>& tabs) {
+    BrickLists b;
     const int na = (int)atom_off.size() - 1, nch = (int)tabs.size(), ng = nch / 4;
-    const int n[3] = {h->nx, h->ny, h->nz};
     b.nbx = (n[0] + kBx - 1) / kBx;
     b.nby = (n[1] + kBy - 1) / kBy;
     const int nbz = (n[2] + kBz - 1) / kBz;
     b.nbricks = b.nbx * b.nby * nbz;
     b.ncg = na * ng;
 
-    // one record per (atom, image, brick): the blocks it covers and where their values are
+    // one record per (atom, image, brick) in order of their first points, and the runs of points in one
+    // block: points [p, p + len) of the atom at x0 .. of block blk in row w of the record's brick
     struct Rec {
         int atom, img, brick;
         u64 mask[8];  // bit 8 b of mask[w]: row w, block b
-        int val[64];
+    };
+    struct Run {
+        int rec, p;
+        unsigned char at, x0, len;  // at = 8 w + blk
     };
     std::vector<Rec> recs;
-    std::vector<double> vals;  // [block of a record][nch][8]
-    std::vector<int> img;      // 3 per image
+    std::vector<Run> runs;
+    runs.reserve(u.size() / 12 + 16);
+    std::vector<int> newest(b.nbricks, -1), before;  // records of a brick, the newest first
     for (int a = 0; a < na; ++a) {
-        std::unordered_map<u64, int> mine;
-        u64 last_key = ~u64(0);
-        int last = -1;
-        for (int p = atom_off[a]; p < atom_off[a + 1]; ++p) {
+        const int first = (int)recs.size();
+        for (int p = atom_off[a]; p < atom_off[a + 1];) {
+            const int* up = &u[3 * (size_t)p];
             int im[3], f[3];
             for (int d = 0; d < 3; ++d) {
-                im[d] = floor_div(u[3 * (size_t)p + d], n[d]);
-                f[d] = u[3 * (size_t)p + d] - im[d] * n[d];
+                im[d] = floor_div(up[d], n[d]);
+                f[d] = up[d] - im[d] * n[d];
             }
+            const int most = std::min({8 - f[0] % 8, n[0] - f[0], atom_off[a + 1] - p});
+            int len = 1;
+            while (len < most && up[3 * len] == up[0] + len && up[3 * len + 1] == up[1] && up[3 * len + 2] == up[2]) ++len;
             int ii = 0;
-            const int ni = (int)img.size() / 3;
-            while (ii < ni && std::memcmp(&img[3 * ii], im, sizeof(im)) != 0) ++ii;
-            if (ii == ni) img.insert(img.end(), im, im + 3);
+            const int ni = (int)b.img.size() / 3;
+            while (ii < ni && std::memcmp(&b.img[3 * ii], im, sizeof(im)) != 0) ++ii;
+            if (ii == ni) b.img.insert(b.img.end(), im, im + 3);
             const int brick = f[0] / kBx + b.nbx * (f[1] / kBy + b.nby * (f[2] / kBz));
-            const u64 key = ((u64)ii << 32) | (u64)brick;
-            if (key != last_key) {
-                auto it = mine.find(key);
-                if (it == mine.end()) {
-                    it = mine.emplace(key, (int)recs.size()).first;
-                    Rec r;
-                    r.atom = a;
-                    r.img = ii;
-                    r.brick = brick;
-                    std::fill(r.mask, r.mask + 8, u64(0));
-                    std::fill(r.val, r.val + 64, -1);
-                    recs.push_back(r);
-                }
-                last_key = key;
-                last = it->second;
+            int r = newest[brick];
+            while (r >= first && recs[r].img != ii) r = before[r];
+            if (r < first) {  // none of this atom
+                r = (int)recs.size();
+                recs.push_back({a, ii, brick, {}});
+                before.push_back(newest[brick]);
+                newest[brick] = r;
             }
-            Rec& r = recs[last];
             const int w = f[1] % kBy, blk = (f[2] % kBz) * 2 + (f[0] % kBx) / 8;
-            int& at = r.val[w * 8 + blk];
-            if (at < 0) {
-                at = (int)(vals.size() / ((size_t)nch * 8));
-                vals.resize(vals.size() + (size_t)nch * 8, 0.0);
-                r.mask[w] |= u64(1) << (8 * blk);
-            }
-            for (int ch = 0; ch < nch; ++ch) vals[((size_t)at * nch + ch) * 8 + f[0] % 8] = tabs[ch][p];
+            recs[r].mask[w] |= u64(1) << (8 * blk);
+            runs.push_back({r, p, (unsigned char)(8 * w + blk), (unsigned char)(f[0] % 8), (unsigned char)len});
+            p += len;
         }
     }
     // records by brick (kept in atom order)
@@ -696,9 +688,10 @@ int build_bricks(qg_hamiltonian h, const std::vector<int>& atom_off, const std::
         std::vector<int> fill(first.begin(), first.end() - 1);
         for (size_t i = 0; i < recs.size(); ++i) order[fill[recs[i].brick]++] = (int)i;
     }
-    std::vector<int> item_brick, item_pair(1, 0), item_cg, item_img, wtab, brick_item(1, 0);
-    std::vector<u64> wmask;
-    std::vector<double> tab;
+    b.item_pair.push_back(0);
+    b.brick_item.push_back(0);
+    size_t ntab = 0;                                    // table blocks of two halves (pairs of groups)
+    std::vector<int> half(recs.size() * ng * 64, -1);   // half of a record's channel group and block
     std::vector<std::vector<int2>> refs(b.ncg);
     auto shared = [](const Rec& p, const Rec& q) {
         int s = 0;
@@ -749,65 +742,80 @@ int build_bricks(qg_hamiltonian h, const std::vector<int>& atom_off, const std::
                 blocks += n;
             }
             b.max_tab = std::max(b.max_tab, blocks);
-            const int item = (int)item_brick.size(), np = (int)(p1 - p0);
+            const int item = (int)b.item_brick.size(), np = (int)(p1 - p0);
             Cg slot[kSlots];
             for (int j = 0; j < 4; ++j) {
                 slot[2 * j] = j < np ? pairs[p0 + j].first : Cg{-1, 0};
                 slot[2 * j + 1] = j < np ? pairs[p0 + j].second : Cg{-1, 0};
             }
-            item_brick.push_back(br);
+            b.item_brick.push_back(br);
             for (int j = 0; j < kSlots; ++j) {
                 const bool on = slot[j].rec >= 0;
                 const int cg = on ? recs[slot[j].rec].atom * ng + slot[j].g : -1;
-                item_cg.push_back(cg);
-                item_img.push_back(on ? recs[slot[j].rec].img : 0);
-                if (on) refs[cg].push_back(make_int2(2 * (item_pair[item] + j / 2) + (j & 1), recs[slot[j].rec].img));
+                b.item_cg.push_back(cg);
+                b.item_img.push_back(on ? recs[slot[j].rec].img : 0);
+                if (on) refs[cg].push_back(make_int2(2 * (b.item_pair[item] + j / 2) + (j & 1), recs[slot[j].rec].img));
             }
             for (int w = 0; w < 8; ++w) {
                 u64 m = 0;
                 for (int j = 0; j < kSlots; ++j)
                     if (slot[j].rec >= 0) m |= recs[slot[j].rec].mask[w] << j;
-                wmask.push_back(m);
-                wtab.push_back((int)(tab.size() / 64));
+                b.wmask.push_back(m);
+                b.wtab.push_back((int)ntab);
                 for (int blk = 0; blk < 8; ++blk)
                     for (int j = 0; j < 4; ++j) {
                         if (!((m >> (8 * blk + 2 * j)) & 3)) continue;
-                        const size_t at = tab.size();
-                        tab.resize(at + 64, 0.0);
                         for (int hf = 0; hf < 2; ++hf) {
                             const Cg& s = slot[2 * j + hf];
-                            if (s.rec < 0) continue;
-                            const int v = recs[s.rec].val[w * 8 + blk];
-                            if (v >= 0)
-                                std::copy_n(&vals[((size_t)v * nch + s.g * 4) * 8], 32, &tab[at + hf * 32]);
+                            if (s.rec >= 0) half[((size_t)s.rec * ng + s.g) * 64 + 8 * w + blk] = (int)(2 * ntab) + hf;
                         }
+                        ++ntab;
                     }
             }
-            item_pair.push_back(item_pair[item] + np);
+            b.item_pair.push_back(b.item_pair[item] + np);
         }
-        brick_item.push_back((int)item_brick.size());
+        b.brick_item.push_back((int)b.item_brick.size());
     }
-    wtab.push_back((int)(tab.size() / 64));
-    b.nitems = (int)item_brick.size();
-    b.npairs = item_pair.back();
-    b.nimg = (int)img.size() / 3;
-    std::vector<int> cg_off(1, 0);
-    std::vector<int2> cg_ref;
+    b.wtab.push_back((int)ntab);
+    // the values: 4 channels x 8 points per half
+    b.tab.resize(ntab * 64, 0.0);
+    for (const Run& r : runs)
+        for (int g = 0; g < ng; ++g) {
+            double* to = &b.tab[(size_t)half[((size_t)r.rec * ng + g) * 64 + r.at] * 32 + r.x0];
+            for (int c = 0; c < 4; ++c) std::copy_n(&tabs[4 * g + c][r.p], r.len, to + 8 * c);
+        }
+    b.nitems = (int)b.item_brick.size();
+    b.npairs = b.item_pair.back();
+    b.nimg = (int)b.img.size() / 3;
+    b.cg_off.push_back(0);
     for (const auto& v : refs) {
-        cg_ref.insert(cg_ref.end(), v.begin(), v.end());
-        cg_off.push_back((int)cg_ref.size());
+        b.cg_ref.insert(b.cg_ref.end(), v.begin(), v.end());
+        b.cg_off.push_back((int)b.cg_ref.size());
     }
-    QG_TRY(upload(&b.item_brick, item_brick));
-    QG_TRY(upload(&b.item_pair, item_pair));
-    QG_TRY(upload(&b.item_cg, item_cg));
-    QG_TRY(upload(&b.item_img, item_img));
-    QG_TRY(upload(&b.wmask, wmask));
-    QG_TRY(upload(&b.wtab, wtab));
-    QG_TRY(upload(&b.brick_item, brick_item));
-    QG_TRY(upload(&b.tab, tab));
-    QG_TRY(upload(&b.cg_off, cg_off));
-    QG_TRY(upload(&b.cg_ref, cg_ref));
-    QG_TRY(upload(&b.img, img));
+    return b;
+}
+
+int upload_bricks(qg_hamiltonian h, const BrickLists& l) {
+    BrickTables& b = h->pj.bricks;
+    b.nbx = l.nbx;
+    b.nby = l.nby;
+    b.nbricks = l.nbricks;
+    b.nitems = l.nitems;
+    b.npairs = l.npairs;
+    b.max_tab = l.max_tab;
+    b.ncg = l.ncg;
+    b.nimg = l.nimg;
+    QG_TRY(upload(&b.item_brick, l.item_brick));
+    QG_TRY(upload(&b.item_pair, l.item_pair));
+    QG_TRY(upload(&b.item_cg, l.item_cg));
+    QG_TRY(upload(&b.item_img, l.item_img));
+    QG_TRY(upload(&b.wmask, l.wmask));
+    QG_TRY(upload(&b.wtab, l.wtab));
+    QG_TRY(upload(&b.brick_item, l.brick_item));
+    QG_TRY(upload(&b.tab, l.tab));
+    QG_TRY(upload(&b.cg_off, l.cg_off));
+    QG_TRY(upload(&b.cg_ref, l.cg_ref));
+    QG_TRY(upload(&b.img, l.img));
     return QG_OK;
 }
 

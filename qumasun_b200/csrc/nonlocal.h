@@ -7,11 +7,20 @@
 
 namespace qg {
 
-// Sphere points of one geometry as the builder takes them: atom a owns the points
+// The lists of BrickTables (qg_internal.h) on the host.
+struct BrickLists {
+    int nbx, nby, nbricks, nitems, npairs, max_tab, ncg, nimg;
+    std::vector<int> item_brick, item_pair, item_cg, item_img, wtab, brick_item, cg_off, img;
+    std::vector<unsigned long long> wmask;
+    std::vector<double> tab;
+    std::vector<int2> cg_ref;
+};
+// From the sphere points of one geometry on a grid of n points per axis: atom a owns the points
 // [atom_off[a], atom_off[a+1]), u = 3 unwrapped grid coordinates per point (rows of
-// consecutive x one after another), tabs[ch][p] the channel values.
-int build_bricks(qg_hamiltonian h, const std::vector<int>& atom_off, const std::vector<int>& u,
-                 const std::vector<std::vector<double>>& tabs);
+// consecutive x one after another), tabs[ch][p] the channel values. No CUDA call.
+BrickLists list_bricks(const int (&n)[3], const std::vector<int>& atom_off, const std::vector<int>& u,
+                       const std::vector<std::vector<double>>& tabs);
+int upload_bricks(qg_hamiltonian h, const BrickLists& l);
 void free_bricks(BrickTables& b);
 
 // Rows of projector coefficients: the count of states (of all k-points) rounded up to 16 (real), or
