@@ -420,8 +420,8 @@ int qg_hamiltonian_test_stall(qg_hamiltonian ham, int on);
 /* Autotuner of the real-state apply (no counterpart in the reference): times, on the
  * caller's DEVICE block of ns states (X in, HX overwritten), the launch shapes that leave
  * every bit of H|psi> unchanged -- stencil kernel (variants 2-5 of
- * qg_hamiltonian_set_stencil_kernel), states per projection block (2, 4, 8, 16) and per
- * scatter group (4, 8) -- one dimension at a time (the phases are independent), best of
+ * qg_hamiltonian_set_stencil_kernel), states per block of the atom-by-atom projection (2, 4,
+ * 8, 16; left alone for FP64 states that are projected brick by brick) and per scatter group (4, 8) -- one dimension at a time (the phases are independent), best of
  * three CUDA-event timed applies each, and keeps the fastest in the operator.
  * choice (3 ints, may be NULL) receives {stencil variant, projection states, scatter
  * states}; ms_phases (3 floats, may be NULL) the chosen configuration's projection,

@@ -4,13 +4,15 @@
 // without changing a single bit of the result: the stencil kernel (one-plane ring,
 // two-plane ring, two rows per thread with V in the ring or from global memory; all give
 // the same sums in the same order), the
-// states per projection block (1-16) and the states per scatter group (4, 8). The split
+// states per block of the atom-by-atom projection (2-16; not where the projection goes by bricks: the
+// operator's value then stays for the calls that use it) and the states per scatter group (4, 8). The split
 // of each atom's projector points over blocks is NOT tuned: it changes the summation
 // order, and results must not depend on the tuning or on the batch. Each phase is
 // timed with CUDA events on the context stream (phase timer of qg_hamiltonian_apply_timed_d:
 // projection, stencil + V, scatter), the best of `reps` applies per candidate; the
-// phases are independent, so each dimension is swept with the others at the engine's
-// choice. The winner is stored in the operator and used by every later apply.
+// phases are taken one after the other (a plain apply runs the stencil beside the atom-by-atom projection
+// and, in small calls, the scatter's start beside the stencil), each dimension with the others at the
+// engine's choice. The winner is stored in the operator and used by every later apply.
 #include <algorithm>
 #include <cfloat>
 #include <vector>
@@ -68,16 +70,18 @@ int autotune(qg_hamiltonian h, int ns, const T* X, long long ldx, T* HX, long lo
     const bool nonlocal = h->pj.na > 0 && h->pj.nch > 0;
     int best_sb = 0, best_sg = 0;
     if (nonlocal) {
-        best_t = FLT_MAX;
-        for (int sb : {2, 4, 8, 16}) {  // projection (phase 0)
-            h->proj_sb = sb;
-            QG_TRY(timed_phases<T>(h, ns, X, ldx, HX, ldhx, reps, ms));
-            if (ms[0] < best_t) {
-                best_t = ms[0];
-                best_sb = sb;
+        if (!qg::real_by_bricks<T>(h)) {  // bricks have no block size to choose
+            best_t = FLT_MAX;
+            for (int sb : {2, 4, 8, 16}) {  // projection (phase 0)
+                h->proj_sb = sb;
+                QG_TRY(timed_phases<T>(h, ns, X, ldx, HX, ldhx, reps, ms));
+                if (ms[0] < best_t) {
+                    best_t = ms[0];
+                    best_sb = sb;
+                }
             }
+            h->proj_sb = best_sb;
         }
-        h->proj_sb = best_sb;
         best_t = FLT_MAX;
         for (int sg : {4, 8}) {  // scatter (phase 2)
             h->scatter_sg = sg;

@@ -207,3 +207,21 @@ def test_small_grids_hold_no_tables_of_point_pairs(cuda_ctx):
     # per sphere point: two orders of 4 channels in FP64 and FP32 and their indices; the bricks' blocks,
     # up to twice as many FP64 values; the potential and per-point rows
     assert taken <= points * (2 * 4 * 12 + 2 * 4 + 2 * 4 * 8) + cell.N * 20 + (12 << 20)
+
+
+def test_autotuner_leaves_a_projection_block_it_does_not_use(cuda_ctx):
+    """FP64 states of more than 16 atoms are projected brick by brick: no block size to choose, and the
+    operator keeps its own for the kernels that have one (FP32 states, the no-allocation entry point)."""
+    import torch
+    from qumasun_b200 import Hamiltonian
+    cell = build_cell(reps=(1, 1, 3), grid=(16, 16, 48))
+    X = torch.from_numpy(initial_states(16, cell.N, seed=6)).cuda()
+    H = Hamiltonian(cuda_ctx, cell)
+    for sb in (0, 1):  # 1: never a candidate
+        H.set_nonlocal_blocking(sb, 0, 0)
+        assert H.autotune(X)["project_states"] == sb
+    H.set_nonlocal_blocking(0, 0, 1)  # atom by atom: the size is used, so it is chosen
+    assert H.autotune(X)["project_states"] in (2, 4, 8, 16)
+    H.set_nonlocal_blocking(0, 0, 0)
+    assert H.autotune(X.float())["project_states"] in (2, 4, 8, 16)
+    H.close()
