@@ -32,12 +32,13 @@ __global__ void k_store_kco(const KcoArgs args, int n, T* __restrict__ out) {
 // Any-shape fallback for V u - 1/2 (Lap + 2i g.grad - g^2) u at FD order 2, 6 or 8: one
 // thread per (point, state), neighbours read from global memory with periodic wrap. The
 // sums follow LaplasianKpoint{2nd,6th,8th}_halo_f (order 2: c0 p + cx (p+x + p-x) + ...;
-// orders 6, 8: c0 p, then the x, y and z groups).
+// orders 6, 8: c0 p, then the x, y and z groups). Runs beside the projection as the ring kernels do.
 template <typename T, int ORDER>
 __global__ void __launch_bounds__(256) k_kpoint_plain(const HamArgs<T> a) {
     constexpr int R = ORDER == 2 ? 1 : (ORDER == 6 ? 3 : 4);
     const long long N = (long long)a.nx * a.ny * a.nz;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    allow_next();
     if (i >= N) return;
     const int s = blockIdx.y;
     const int ix = (int)(i % a.nx), iy = (int)((i / a.nx) % a.ny), iz = (int)(i / ((long long)a.nx * a.ny));
@@ -99,6 +100,7 @@ __global__ void __launch_bounds__(256) k_kpoint_plain(const HamArgs<T> a) {
     T* h = a.HX + state_offset(a, s, true) + i;
     h[0] = (v * cen[0] + lap[0]) - der[1];
     h[a.hxim] = (v * cen[1] + lap[1]) + der[0];
+    wait_previous();
 }
 
 // c0 and the first-derivative coefficients of -1/2 (Lap + 2i g.grad - g^2) at FD order
@@ -204,11 +206,8 @@ int apply_hamiltonian_zk(qg_hamiltonian h, int nk, const double* kv, int nsk, co
     auto stencil = [&](bool early) -> int {
         if (plain) {
             dim3 g((unsigned)((N + 255) / 256), (unsigned)(nk * nsk));
-            switch (h->order) {
-                case 2: k_kpoint_plain<T, 2><<<g, 256, 0, st>>>(a); break;
-                case 6: k_kpoint_plain<T, 6><<<g, 256, 0, st>>>(a); break;
-                default: k_kpoint_plain<T, 8><<<g, 256, 0, st>>>(a); break;
-            }
+            auto kern = h->order == 2 ? k_kpoint_plain<T, 2> : (h->order == 6 ? k_kpoint_plain<T, 6> : k_kpoint_plain<T, 8>);
+            QG_CUDA_TRY(launch_kernel(early, kern, g, dim3(256), 0, st, a));
             return QG_OK;
         }
         a.early = early;
@@ -224,7 +223,7 @@ int apply_hamiltonian_zk(qg_hamiltonian h, int nk, const double* kv, int nsk, co
     if (pt) pt->mark(1, st);
     if (!together) QG_TRY(stencil(false));
     if (pt) pt->mark(2, st);
-    if (nonlocal) QG_TRY(brick_scatter_z<T>(h, nk, nsk, HX, ldhx, ldkh, phase, scratch, together && !plain && small_call((long long)nk * nsk * N), st));
+    if (nonlocal) QG_TRY(brick_scatter_z<T>(h, nk, nsk, HX, ldhx, ldkh, phase, scratch, together && small_call((long long)nk * nsk * N), st));
     if (pt) pt->mark(-1, st);
     QG_CUDA_TRY(cudaGetLastError());
     return QG_OK;

@@ -128,14 +128,16 @@ struct LanePhase {
     }
 };
 
-// The item's table into shared memory, 16 bytes per thread and step; waits.
-__device__ __forceinline__ void load_table(double* tb, const BrickGeom& g, int item) {
+// The item's table into shared memory, 16 bytes per thread and step; table_ready waits for it.
+__device__ __forceinline__ void fetch_table(double* tb, const BrickGeom& g, int item) {
     const int w0 = g.wtab[item * 8], w1 = g.wtab[item * 8 + 8];
     const double* src = g.tab + (long long)w0 * 64;
     for (int i = threadIdx.x; i < (w1 - w0) * 32; i += kThreads)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(tb + 2 * i)),
                      "l"(src + 2 * i)
                      : "memory");
+}
+__device__ __forceinline__ void table_ready() {
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 }
@@ -155,6 +157,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     constexpr int S = CPLX ? 2 : 1;
     extern __shared__ __align__(16) double tb[];
     __shared__ double red[ROWS ? 8 : 1][ROWS ? S * 4 * 64 : 1];
+    allow_next();
     const int chunks = ROWS ? nunit : (nunit + 7) / 8;
     const int item = blockIdx.x / chunks, ch = blockIdx.x - item * chunks;
     const int brick = g.item_brick[item];
@@ -182,7 +185,8 @@ __global__ void __launch_bounds__(kThreads, 2)
     u64 mn = g.wmask[item * 8 + row_a];
 #pragma unroll
     for (int d = 0; d < D - 1; ++d) fetch(mn, row_a, d, a[d]);
-    load_table(tb, g, item);
+    fetch_table(tb, g, item);
+    table_ready();
     const double* tp = tb + (g.wtab[item * 8 + row_a] - g.wtab[item * 8]) * 64 + 2 * lane;
 
     double tot[S][4][2];
@@ -334,8 +338,13 @@ __global__ void __launch_bounds__(kThreads, 2)
     const double2* ph = phase + (long long)k * nphase;
     const int row_a = ROWS ? w : 0, row_b = ROWS ? w + 1 : 8;
     using P2 = typename Pair<T>::type;
+    // Few units, where latency counts: the table, which no kernel before this one writes, on its way before the
+    // wait (one complex64 state of 41^3 29.6 -> 28.7 us a call; for many units behind the loads that are used
+    // first, 64 complex128 states of 80^3 0.4 % faster so).
+    const int first = g.brick_item[brick], last = g.brick_item[brick + 1];
+    if (ROWS && first < last) fetch_table(tb, g, first);
     wait_previous();
-    for (int item = g.brick_item[brick]; item < g.brick_item[brick + 1]; ++item) {
+    for (int item = first; item < last; ++item) {
         P2 hv[D][2];
         auto fetch = [&](u64 m, int row, int b, P2 (&v)[2]) {
             if ((m >> (8 * b)) & 255) {
@@ -363,7 +372,8 @@ __global__ void __launch_bounds__(kThreads, 2)
                 A[j][1] = p.x * im - p.y * re;
             }
         }
-        load_table(tb, g, item);
+        if (!ROWS || item > first) fetch_table(tb, g, item);
+        table_ready();
         const double* tp = tb + (g.wtab[item * 8 + row_a] - g.wtab[item * 8]) * 64 + q * 8 + r;
         LanePhase lp;
         for (int row = row_a; row < row_b; ++row) {

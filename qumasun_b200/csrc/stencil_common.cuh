@@ -8,12 +8,13 @@ namespace qg {
 
 // Overlap of the kernels of an operator application (programmatic dependent launch). The projection
 // and the stencil read the same states and write different buffers: the projection lets the next kernel
-// of its stream start at once (allow_next), the stencil starts beside it and ends only after it
-// (wait_previous, last thing), so that whatever follows the stencil follows both. In small calls the
+// of its stream start as soon as its own last blocks have (allow_next), the stencil starts beside it and ends
+// only after it (wait_previous, last thing), so that whatever follows the stencil follows both. In small calls the
 // kernels after the stencil start early too, read their tables and then wait (wait_previous): large calls
 // lose by that, blocks that come onto an SM beside the stencil's keep its shared-memory split and little
 // L1 (256 states of 80^3: the scatter 0.65 ms instead of 0.44). 16 states of 40^3: 36.9 us per call one
-// after another, 31.0 so; one state of 36^3 34 and 26.
+// after another, 31.0 so; one complex64 state of 40^3 41.1 with the brick projection before the stencil, 34.9
+// beside it; 64 states of 80^3 399 and 389 (256: the same within the noise).
 __device__ __forceinline__ void allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
