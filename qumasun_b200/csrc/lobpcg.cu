@@ -1149,8 +1149,10 @@ int run_lobpcg_zk(qg_hamiltonian h, const qg_lobpcg_options* opt, int nk, const 
         s.lwork = std::max(lw1, lw2);
         QG_TRY(s.work.reserve((size_t)std::max(s.lwork, 1) * sizeof(cuDoubleComplex)));
     }
-    QG_TRY(h->coef.reserve(qg::kpoint_scratch(h, nk, nb)));
-    if (2 * nb <= qg::kGramTsMax) QG_TRY(s.gts.reserve(qg::gram_ts_scratch_doubles(N, nk, true) * sizeof(double)));
+    // the operator's scratch, between its applications also the partial sums of the tall-skinny Gram products
+    // (compact: 2 nb x 2 nb each): the operator keeps it, a buffer of the solve is allocated and freed by every call
+    const size_t gram_part = 2 * nb <= qg::kGramTsMax ? (size_t)nk * qg::gram_ts_blocks(N, nk) * 2 * 4 * nb * nb : 0;
+    QG_TRY(h->coef.reserve(std::max(qg::kpoint_scratch(h, nk, nb), gram_part * sizeof(double))));
     // pencils of up to kSmallHegMax rows: all k-points' Hermitian pencils in one launch
     // of the one-block Jacobi solver (small_eig.cu), cuSOLVER's zhegvd per k-point
     // otherwise and for any pencil the Jacobi solver rejects
@@ -1188,7 +1190,7 @@ int run_lobpcg_zk(qg_hamiltonian h, const qg_lobpcg_options* opt, int nk, const 
                          int g) -> int {
         if (2 * nb <= qg::kGramTsMax)
             return qg::gram_ts(Wi, N, kstride, AWj, Wj, N, kstride, N, 2 * nb, 2 * nb, s.dV, Ca_, Cb_, g, (long long)gsz,
-                               nk, s.gts.as<double>(), st);
+                               nk, h->coef.as<double>(), st);
         const double zero = 0.0;
         for (int k = 0; k < nk; ++k) {
             const double* A = Wi + k * kstride;
