@@ -127,7 +127,10 @@ int qg_hamiltonian_set_kvector(qg_hamiltonian ham, double gx, double gy, double 
 
 /* HX[s] = H X[s] for ns states, DEVICE pointers, FP64.
  * Replaces ns calls of OpeA -> mHamiltonianMatrix(_ddm) (qumasun_single.matrix.h:19-40,
- * qumasun_mpi.matrix.h:20-43) and the bundled mHamiltonianMatrix_bundle_ddm (:46-104). */
+ * qumasun_mpi.matrix.h:20-43) and the bundled mHamiltonianMatrix_bundle_ddm (:46-104).
+ * A NaN or Inf stays in its own state, but in all applications it can reach more points of it
+ * than the stencil and the spheres alone: projections take blocks of 8 consecutive x (0 * NaN;
+ * FP64 states of more than 16 atoms, all complex states), the scatter pairs of points. */
 int qg_hamiltonian_apply_d(qg_hamiltonian ham, int ns, const double* X, long long ldx,
                            double* HX, long long ldhx);
 /* Same in FP32 (float states; V and projector tables rounded from FP64 once). */
@@ -184,7 +187,9 @@ int qg_hamiltonian_apply_timed_d(qg_hamiltonian ham, int ns, const double* X, lo
                                  double* HX, long long ldhx, float* ms_phases);
 /* No counterpart in the reference (its CPU operator allocates freely).
  * Same result as qg_hamiltonian_apply_d (FP64, DEVICE pointers, context
- * stream), for callers that cannot call cudaMalloc at the point of the call:
+ * stream) -- the same bits for cells of at most 16 atoms, up to the last bits of the
+ * projections above, which this call always sums atom by atom (the array does not hold
+ * the sums of the brick projection) -- for callers that cannot call cudaMalloc at the point of the call:
  * hosts whose device memory belongs to another framework's allocator (a pool
  * that must not be bypassed), and time-critical loops that must not touch the
  * allocator. It allocates nothing: the projector coefficients go to a scratch
@@ -280,9 +285,10 @@ int qg_lobpcg_z(qg_hamiltonian ham, const qg_lobpcg_options* opt, int ns, double
  * qg_lobpcg_z once per k-point): kvecs = nk Bloch vectors (HOST, 3 each), nsk states
  * per k-point, X and P DEVICE, [k][s] state-major ({re[N], im[N]} per state), ev HOST
  * (nk * nsk). H, norms, residuals and the preconditioner run over all k-points' states in
- * single launches; Gram products are DGEMMs per k-point, rotations strided-batched DGEMMs
- * over k; the nsk-state pencils are solved k-point by k-point, and a k-point whose states
- * have converged is frozen (no further rotation or solve). FP64; precond 0 or 1; stops when the
+ * single launches; Gram products of up to 32 states per k-point run for all k-points in one
+ * launch, of more as DGEMMs per k-point, rotations are strided-batched DGEMMs over k; pencils
+ * of up to 56 rows are solved in one launch, larger ones k-point by k-point, and a k-point
+ * whose states have converged is frozen (no further rotation or solve). FP64; precond 0 or 1; stops when the
  * lowest n_converge states of every k-point meet tol. The report carries iterations,
  * convergence, max_residual, ms_total and restarts. No counterpart in the reference,
  * which loops over k-points (qumasun_kpoint.lobpcg.h:25-41). */
@@ -388,8 +394,8 @@ int qg_hegv_small_batched_z(qg_context ctx, int batch, int k, const double* A, c
  * 1 = always the register-window kernel (any shape), 2 = the one-plane ring
  * kernel, 3 = the two-plane ring kernel, 4 = the ring kernel with two grid rows per
  * thread and V streamed through the ring, 5 = the same with V read one plane ahead from
- * global memory (2-5 fall back as 0 does where the shape does not fit). All give the same bits. Complex states use the one-plane ring kernel
- * unless 1 is set. */
+ * global memory (2-5 fall back as 0 does where the shape does not fit). All give the same
+ * bits. Complex states have a ring kernel of their own, 1 selects their any-shape kernel. */
 int qg_hamiltonian_set_stencil_kernel(qg_hamiltonian ham, int variant);
 /* Tuning of the nonlocal passes of real states: states per block of the atom-by-atom
  * projection (1, 2, 4, 8 or 16), states per scatter group (4 or 8), and blocks per atom
@@ -481,8 +487,8 @@ int qg_potential_lda_d(qg_poisson p, const double* rho, const double* pcc, const
 
 /* One fourth-order Taylor step psi <- sum_{j=0..4} (-i dt H)^j / j! psi of ns complex
  * {re[N], im[N]} states (DEVICE, in place, ldx >= 2N) under the operator at its
- * k-vector (FD order 2, 6 or 8): four applications of H to the whole block, each followed by
- * the update of that order. Work: two blocks of ns states kept by the operator.
+ * k-vector (FD order 2, 6 or 8): four applications of H to the whole block, each two followed by
+ * the update of both orders. Work: two blocks of ns states kept by the operator.
  * Replaces QUMASUN::TimeEvoH4 (qumasun_td.time_evo_H4.h:13-60), which steps one state
  * at a time. */
 int qg_td_taylor4_z(qg_hamiltonian ham, int ns, double dt, double* X, long long ldx);
@@ -495,7 +501,8 @@ int qg_td_taylor4_z(qg_hamiltonian ham, int ns, double dt, double* X, long long 
  * sum E inner dinner_d; *ev_sum = sum occ[s] e_state[s]. occ, forces (3 per atom,
  * accumulated), e_state (may be NULL) and ev_sum (may be NULL) are HOST. QG_ERR_TIMEOUT (a
  * bounded wait on the device ran out, here or in an earlier launch) leaves forces and e_state
- * as they were. Replaces
+ * as they were. A NaN or Inf in a state reaches the gradient's whole 8 x 8 tiles of x and y.
+ * Replaces
  * QUMASUN_MPI::mGetForcePseudoNonlocal (qumasun_mpi.force.h:227-254) with
  * PseudoPotIntegrator_mpi::ForceNonlocal (PseudoPotOperator_mpi_v2.h:905-1010). */
 int qg_nonlocal_force_d(qg_hamiltonian ham, int ns, const double* X, long long ldx, const double* occ,

@@ -10,7 +10,7 @@
 // neighbour -- the accumulator layout of m8n8k4. Per plane: 16 inputs of 8 outputs in four steps
 // along x (band on the right) and along y (band on the left), the z difference from the 9 values of
 // each point in registers, which rotate by renaming. Bound: DRAM, 8 bytes in and 24 out per point;
-// 139 of 256 states of 80^3 take 0.53 ms (0.35 ms of bytes at the copy rate), against 4.0 ms for
+// 139 of 256 states of 80^3 take 0.49 ms (0.35 ms of bytes at the copy rate), against 4.0 ms for
 // 24 neighbour loads per point from L1 (k_gradient8, which stays for the shapes TMA does not take).
 // The same products in the Hamiltonian's stencil measured slower than its vector kernels (1.17
 // against 0.55 ms real, 0.63 against 0.44 k-points): the FP64 tensor and vector instructions share

@@ -130,8 +130,10 @@ __global__ void __launch_bounds__(TV) k_conv_fwd(const TI* __restrict__ in, cons
 // ---------------- backward pass on the tensor cores (mma.sync m16n8k16, BF16 in, FP32 sums)
 // The FP32 gradients enter as three BF16 pieces (d = d1 + d2 + d3 to 2^-24 of d or 5e-41), the activations and
 // weights are BF16 already, so the products are those of the FP32 kernels; the FP32 sums of a
-// tile are added to the running sums with ordinary rounding. Bound: shared-memory reads of the
-// operands (ldmatrix); one layer of 16 x 16 channels at 32 states of 40^3 is 14 G multiply-adds.
+// tile are added to the running sums with ordinary rounding. Bound: k_dgrad_mma the shared-memory reads of the
+// operands (ldmatrix, 80 % of L1), k_wgrad_mma the tensor pipe (44 %) and, before it in every tile, the loads
+// that stage the tile; one layer of 16 x 16 channels at 32 states of 40^3 is 14 G multiply-adds: 0.43
+// and 0.35 ms.
 // Operand tiles are [voxel][16 channels], 32 bytes a voxel; the two 16-byte halves of a voxel
 // change places every 4 voxels, so the 8 rows of any ldmatrix fall into different banks.
 __device__ __forceinline__ int half_at(int v, int h) { return (2 * v + (h ^ ((v >> 2) & 1))) * 8; }  // in elements

@@ -28,9 +28,9 @@
 //
 // Measured, projection (with its sums) / scatter: 64 complex128 states of 80^3 0.26 / 0.28 ms
 // (atom by atom and point by point: 0.41 / 0.33), 64 k-points x 16 complex64 states of 40^3
-// 0.46 / 0.51 (0.58 / 0.61); real FP64, 256 states of 80^3 0.36 ms against 0.49, 528 of 120^3 2.70
+// 0.42 / 0.39 (0.58 / 0.61); real FP64, 256 states of 80^3 0.36 ms against 0.49, 528 of 120^3 2.71
 // against 3.71, where the atom-by-atom kernel reads psi 2.65 times from DRAM. Real states keep
-// their point-by-point scatter (0.52 ms; this form 0.68) and FP32 the atom-by-atom projection
+// their scatter by pairs of points (0.44 ms; this form 0.68) and FP32 the atom-by-atom projection
 // (0.31; 0.34): there the 64- and 32-byte pieces of a load limit the bricks.
 //
 // A state with a NaN or Inf at a point spreads it to every sphere that meets the point's block
@@ -147,8 +147,10 @@ __device__ __forceinline__ void table_ready() {
 // warps take one row of the brick each for one unit (few units: more warps per state);
 // otherwise they take one unit each and walk the whole brick, the table in shared memory. Both
 // add a row's blocks first and then the rows in order, so the sums are the same to the bit.
-// Bound: the FP64 tensor pipe (58 % busy) and the 64-byte pieces of the loads (3.1 TB/s of psi);
-// D blocks of states are in flight per warp.
+// Bound: the FP64 tensor pipe (65 % busy for real, 50 for complex128, 58 for complex64 states) and the
+// 64-byte pieces of the loads (3.2 TB/s of psi at 64 real states of 80^3); D blocks of states are in flight per
+// warp. Two blocks per SM leave 128 registers, where the complex forms that walk the whole brick spill 28 to 84
+// bytes.
 template <typename T, bool CPLX, bool VEC, bool ROWS, int D>
 __global__ void __launch_bounds__(kThreads, 2)
     k_brick_project(const T* __restrict__ X, long long ldx, long long ldk, long long xim, int ns, int nrow,

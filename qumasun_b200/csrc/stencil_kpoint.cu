@@ -14,7 +14,8 @@
 // Bound: latency. 11 (FP64) or 15 (FP32) warps are what the z-windows leave room for; the FP64 pipe is
 // 48 %, the issue slots 48 %, L1 45 % and L2 16 % busy. A thread with both parts of a point (two windows,
 // 168 registers with spills, 10 warps) took 0.66 ms for 64 complex128 states of 80^3 and 1.22 ms for 64
-// k-points x 16 complex64 states of 40^3; this one 0.44 and 0.62 ms. One row per thread: 0.51 / 0.75.
+// k-points x 16 complex64 states of 40^3; this one 0.44 and 0.62 ms (0.65 where it starts beside the projection's
+// last blocks). One row per thread: 0.51 / 0.75.
 // Every wait is bounded (QG_ERR_TIMEOUT in the device status word on expiry).
 #include <algorithm>
 #include <cstdint>
@@ -62,8 +63,11 @@ __device__ __forceinline__ void add_pair(T& lap, T& der, T p, T m, T w, int i) {
     der += T(der_ratio<ORDER>(i)) * (p - m);
 }
 
-// NXC > 0: the row length as a compile-time constant (the common grids), which makes the
-// y-neighbour offsets immediates of the shared-memory loads.
+// NXC > 0: the row length as a compile-time constant, which makes the y-neighbour offsets immediates of the
+// shared-memory loads; the row lengths of the synthetic cells (40 points per 8-atom cell edge), as in the
+// other ring kernels. Order 8, without / with: 256 complex64 states of 40^3 239 / 214 us, 64 of 80^3 433 / 350, 64
+// complex128 states of 80^3 574 / 485, 16 of 120^3 523 / 439 (order 6: 193 / 190, -, 441 / 405). All other lengths run
+// without.
 template <typename T, int ORDER, int NXC, int RPT>
 __global__ void __launch_bounds__(kConsumers<T> + 32, 1) k_stencil_kpoint(const HamArgs<T> a, const WorkGrid wg, int nst) {
     constexpr int PX = 16 / sizeof(T);

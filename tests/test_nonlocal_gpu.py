@@ -225,3 +225,20 @@ def test_autotuner_leaves_a_projection_block_it_does_not_use(cuda_ctx):
     H.set_nonlocal_blocking(0, 0, 0)
     assert H.autotune(X.float())["project_states"] in (2, 4, 8, 16)
     H.close()
+
+
+@pytest.mark.parametrize("reps,same", [((1, 1, 1), True), ((2, 1, 1), True), ((3, 1, 1), False)])
+def test_noalloc_entry_sums_atom_by_atom(cuda_ctx, reps, same):
+    """The no-allocation entry point: the regular one's bits up to 16 atoms, above them another order of the
+    projections' sums (a few thousand terms: the bound of the other operator tests), whatever the batch."""
+    import torch
+    from qumasun_b200 import Hamiltonian
+    cell = build_cell(reps=reps, grid=(20 * reps[0], 18, 16), displacement=0.05, seed=2)
+    X = torch.from_numpy(initial_states(9, cell.N, seed=4)).cuda()
+    H = Hamiltonian(cuda_ctx, cell)
+    ref, out = H.apply(X), H.apply_noalloc(X, torch.empty_like(X))
+    assert torch.equal(out, ref) if same else ((out - ref).norm(dim=1) < 1e-12 * ref.norm(dim=1)).all()
+    H.set_nonlocal_blocking(0, 0, 1 if not same else 0)  # the regular entry's atom-by-atom form
+    assert torch.equal(H.apply(X), out)
+    assert torch.equal(H.apply_noalloc(X[8:], torch.empty_like(X[8:])), out[8:])
+    H.close()
