@@ -188,8 +188,8 @@ int qg_hamiltonian_apply_timed_d(qg_hamiltonian ham, int ns, const double* X, lo
 /* No counterpart in the reference (its CPU operator allocates freely).
  * Same result as qg_hamiltonian_apply_d (FP64, DEVICE pointers, context
  * stream) -- the same bits for cells of at most 16 atoms, up to the last bits of the
- * projections above, which this call always sums atom by atom (the array does not hold
- * the sums of the brick projection) -- for callers that cannot call cudaMalloc at the point of the call:
+ * projections above, which this call always sums atom by atom (the array is too small
+ * for the brick projection's sums in large cells) -- for callers that cannot call cudaMalloc at the point of the call:
  * hosts whose device memory belongs to another framework's allocator (a pool
  * that must not be bypassed), and time-critical loops that must not touch the
  * allocator. It allocates nothing: the projector coefficients go to a scratch
