@@ -21,6 +21,7 @@
 #include <cstring>
 #include <functional>
 #include <future>
+#include <new>
 #include <vector>
 
 #include <cooperative_groups.h>
@@ -892,7 +893,7 @@ int build_projectors(qg_hamiltonian h, const qg_hamiltonian_desc* d) {
         for (int k = 0; k < np; ++k)
             for (int m = 0; m < 2 * d->proj_l[k] + 1; ++m) { ch_k[c] = k; ch_m[c] = m; ++c; }
     }
-    size_t most = 0;  // points of the cubes: room for every one, of which the pages that hold points are touched
+    size_t most = 0;  // points of the cubes: room for all (3 GB at most), of which the pages that hold points are touched
     for (int a = 0; a < na; ++a) {
         size_t cube = 0;
         for (int k = 0; k < np; ++k) {
@@ -901,6 +902,7 @@ int build_projectors(qg_hamiltonian h, const qg_hamiltonian_desc* d) {
         }
         most += cube;
     }
+    most = std::min(most, size_t(1) << 26);
     pt_g.reserve(most);
     pt_u.reserve(3 * most);
     for (auto& t : tabs) t.reserve(most);
@@ -1069,11 +1071,16 @@ int qg_hamiltonian_create(qg_context ctx, const qg_hamiltonian_desc* d, qg_hamil
     h->gx = d->gx; h->gy = d->gy; h->gz = d->gz;
     h->ty = ty;
     const long long N = h->N();
-    std::vector<double> V(d->V, d->V + N);
-    std::vector<float> Vf(V.begin(), V.end());
-    int rc = upload(&h->V_d, V);
-    if (rc == QG_OK) rc = upload(&h->V_f, Vf);
-    if (rc == QG_OK) rc = build_projectors(h, d);
+    int rc;
+    try {
+        std::vector<double> V(d->V, d->V + N);
+        std::vector<float> Vf(V.begin(), V.end());
+        rc = upload(&h->V_d, V);
+        if (rc == QG_OK) rc = upload(&h->V_f, Vf);
+        if (rc == QG_OK) rc = build_projectors(h, d);
+    } catch (const std::bad_alloc&) {  // host tables, here or in the thread that lists the bricks
+        rc = QG_ERR_NOMEM;
+    }
     if (rc != QG_OK) {
         destroy_ham(h);
         return rc;
