@@ -487,12 +487,15 @@ int launch_project(qg_hamiltonian h, int nk, int ns, const T* X, long long ldx, 
         const long long prow = (long long)nu * (CPLX ? 16 : 8);
         kern<<<(unsigned)((long long)b.nitems * (ROWS ? nu : (nu + 7) / 8)), kThreads, (size_t)b.max_tab * 512, st>>>(
             X, ldx, ldk, h->N(), ns, nrow, u0, nu, geom(h), phase, np, part, prow);
-        // one slice: the stencil runs beside the projection, and ends after it
-        const bool beside = stencil && nu == units;
-        if (beside) QG_TRY(stencil(true));
-        QG_CUDA_TRY(launch_kernel(beside && small_call((long long)nk * ns * h->N()), k_brick_reduce<CPLX>, dim3(b.ncg, nu),
-                                  dim3(kThreads), 0, st, part, prow, b.cg_off, b.cg_ref, ns, nrow, u0, phase, np,
-                                  h->nx + h->ny + h->nz, scale, coef, coef_rows(nrow, CPLX)));
+        // one slice: the stencil runs beside the projection, in small calls of few units beside the sums as well, and
+        // ends after them (16 complex64 states of 40^3 53.1 -> 48.1 us a call, 8 real ones of 64 atoms on 80^3 100.9 ->
+        // 94.4; 64 complex64 states of 40^3, 8 units, 157 -> 169: blocks of the sums keep the stencil off their SMs)
+        const bool beside = stencil && nu == units, small = ROWS && small_call((long long)nk * ns * h->N());
+        if (beside && !small) QG_TRY(stencil(true));
+        QG_CUDA_TRY(launch_kernel(beside && small_call((long long)nk * ns * h->N()), k_brick_reduce<CPLX>, dim3(b.ncg, nu), dim3(kThreads), 0, st, part, prow,
+                                  b.cg_off, b.cg_ref, ns, nrow, u0, phase, np, h->nx + h->ny + h->nz, scale, coef,
+                                  coef_rows(nrow, CPLX)));
+        if (beside && small) QG_TRY(stencil(true));
     }
     if (stencil && units > most) QG_TRY(stencil(false));
     QG_CUDA_TRY(cudaGetLastError());

@@ -14,7 +14,8 @@ namespace qg {
 // lose by that, blocks that come onto an SM beside the stencil's keep its shared-memory split and little
 // L1 (256 states of 80^3: the scatter 0.65 ms instead of 0.44). 16 states of 40^3: 36.9 us per call one
 // after another, 31.0 so; one complex64 state of 40^3 41.1 with the brick projection before the stencil, 34.9
-// beside it; 64 states of 80^3 399 and 389 (256: the same within the noise).
+// with the stencil beside it, 30.5 beside its sums too; 64 states of 80^3 399 and 389 (256: the same within the
+// noise).
 __device__ __forceinline__ void allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
